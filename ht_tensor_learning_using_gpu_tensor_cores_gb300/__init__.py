@@ -204,7 +204,8 @@ def decompose(x, tree: DimTree, dims: Optional[Sequence[int]] = None, precision:
     """HT decomposition of a column-major 3rd/4th-order float32 tensor.
 
     precision="bf16": BF16 tcgen05 GEMMs with FP32 accumulation (the mixed path);
-    precision="fp32": every product in FP32 on CUDA cores (the plain path).
+    precision="fp32": every product to FP32 accuracy (the plain path: CUDA cores,
+    or three BF16 planes per operand on tensor cores).
     eig_iters: subspace iterations of the leaf solver (0: 10 on FP32, 6 on BF16).
     leaf_method="gram": leaf bases from the mode Grams (subspace iteration,
     eig_iters); "sketch": from the Gram-free range finder on X_(t)

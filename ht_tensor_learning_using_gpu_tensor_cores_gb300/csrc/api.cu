@@ -200,6 +200,17 @@ struct Ctx {
   int launches = 0;
   int path = 0;         // bit 0 tcgen05, bit 1 SIMT
   bool tc = false;
+  // FP32 products as three-plane BF16 splits on tcgen05 (tc3_gemm.cu), where
+  // the call's workspace holds the planes; off: CUDA cores
+  bool tc3 = false;
+  // X's planes (first mode padded to x3_n1p rows), set by enqueue_body
+  const __nv_bfloat16 *x3 = nullptr;
+  long long x3_plane = 0;
+  long x3_n1p = 0;
+  // entries without planes (not finite): *nf == epoch makes the guarded FP32
+  // kernel form the product again (null: the caller rejects such data itself)
+  int *nf = nullptr;
+  int epoch = 0;
   int eig_ctas = 0;     // cap on the cooperative eigen-solver's grid (0 = every SM)
   // Staged enqueue of the batched path.  eig_mode 0: leaf_eigs launches the
   // cooperative solver; 1: it appends its problems to eig_table (the grouped
@@ -260,6 +271,7 @@ Operand gram_operand(const View &v, const void *x) {
 int sm_count() { return device_sm_count(); }
 
 struct GemmReq {
+  GemmReq() { a16.ptr = b16.ptr = a3.ptr = b3.ptr = nullptr; }
   Operand a32, b32;                 // FP32 operands (SIMT path)
   Operand a16, b16;                 // BF16 operands (tcgen05 path); ptr null = unavailable
   int bn_tc = 128, bn_simt = 128;
@@ -276,6 +288,10 @@ struct GemmReq {
   bool fold = false;                // tcgen05 only: b16 is a high/low split (GemmArgs::fold)
   int mt_tc = 1;                    // tcgen05 only: 2 = 256-row tiles (GemmArgs::mt)
   __nv_bfloat16 *out16 = nullptr;   // column-major output wanted in BF16 here (q.out may then be scratch)
+  Operand a3, b3;                   // three-plane operands (Ctx::tc3); ptr null = unavailable
+  long long a3_plane = 0, b3_plane = 0;
+  const float *bias = nullptr;      // row bias and ReLU of a column-major output
+  bool relu = false;
   // split-K partials into the caller's buffer with exactly force_splits
   // splits, no reduction (the caller reduces several launches' partials at once)
   float *part_ext = nullptr;
@@ -284,7 +300,10 @@ struct GemmReq {
 
 // D = A B^T over the tiles: tcgen05 on the BF16 operands when the context
 // allows it and the shapes map to TMA, else SIMT on the FP32 operands.
+ht_status_t run_gemm3(Ctx &c, const GemmReq &q);
 ht_status_t run_gemm(Ctx &c, const GemmReq &q) {
+  if (c.tc3 && q.a3.ptr && q.b3.ptr && tc3_supported(q.a3, q.a3_plane, q.b3, q.b3_plane))
+    return run_gemm3(c, q);
   bool use_tc = c.tc && q.a16.ptr && q.b16.ptr;
   if (use_tc) {
     GemmArgs probe;
@@ -400,6 +419,9 @@ ht_status_t run_gemm(Ctx &c, const GemmReq &q) {
   // from the FP32 result converted afterwards
   const bool direct16 = q.out16 && use_tc && !partial;
   g.out16 = direct16 ? q.out16 : nullptr;
+  const bool fused = use_tc && !partial;   // the tcgen05 epilogue adds the bias itself
+  g.bias = fused ? q.bias : nullptr;
+  g.relu = fused && q.relu ? 1 : 0;
   if (use_tc) {
     HT_CUDA(tc_gemm_launch(g, bn, c.st));
     c.path |= 1;
@@ -413,11 +435,119 @@ ht_status_t run_gemm(Ctx &c, const GemmReq &q) {
                                    (q.symmetric ? 1 : 0) | (q.accumulate ? 2 : 0), c.st));
     ++c.launches;
   }
+  if (!fused && (q.bias || q.relu)) {   // y row-major = this output's columns
+    HT_CUDA(bias_act_launch(q.out, q.bias, q.t_n, q.ld_out, q.relu ? 1 : 0, c.st));
+    ++c.launches;
+  }
   if (q.out16 && !direct16) {   // rows x cols column-major, ld = rows
     HT_CUDA(f32_to_bf16_launch(q.out, q.out16, q.ld_out * q.t_cols, c.st));
     ++c.launches;
   }
   c.ar.off = mark;   // scratch is stream-ordered: later work may reuse it
+  return HT_OK;
+}
+
+// D = A B^T to FP32 accuracy from the operands' BF16 planes.
+//
+// Tile columns: the widest tile reads the fewest operand bytes per MMA and was
+// the fastest at every Gram and layer size measured (1024 x 8192 x 1024: 97 us
+// at 256, 130 at 128, 240 at 64; Grams of 260 to 397: 145 us against 198 at 64
+// although the 256-wide tiles compute 2.3 x the outputs), except where its tiles
+// are too few for the SMs and K too short to split: then narrower ones spread
+// the work.  Splits keep at least 16 K blocks each, so that the ring fills and a
+// short product needs no reduction launch.
+ht_status_t run_gemm3(Ctx &c, const GemmReq &q) {
+  TileGen gen;
+  auto make = [&](int bn) {
+    if (q.tiles_kind == TILES_ROWS) gen = make_rows_gen(q.t_rows, q.t_cols, bn);
+    else if (q.tiles_kind == TILES_SLABS) gen = make_slabs_gen(q.t_L, q.t_R, q.t_cols, bn);
+    else if (q.tiles_kind == TILES_GRID) return make_grid_gen(q.t_rows, q.t_n, bn, &gen);
+    else return make_gram_gen(q.t_n, bn, &gen, 128);
+    return true;
+  };
+  const long nkb = tc3_num_kblocks(q.a3);
+  const long long width = q.tiles_kind == TILES_GRID || q.tiles_kind == TILES_GRAM ? q.t_n : q.t_cols;
+  int bn = 256;
+  for (;; bn /= 2) {
+    if (!make(bn)) return fail(HT_ERR_UNSUPPORTED, "product too large for one grid");
+    if (bn == 64) break;
+    const long long work = gen.count * std::max<long long>(1, q.allow_split ? nkb / 16 : 1);
+    if (width > bn / 2 && 2 * work >= sm_count()) break;
+  }
+  const int nt = gen.count;
+  int splits = 1;
+  if (q.force_splits > 0) splits = q.force_splits;
+  else if (q.allow_split && nt < sm_count()) {
+    splits = std::max(1, sm_count() / nt);
+    long per = (nkb + splits - 1) / splits;
+    per = std::max<long>(per, std::min<long>(nkb, 16));
+    splits = static_cast<int>((nkb + per - 1) / per);
+  }
+  const bool partial = splits > 1 || q.out_mode == OUT_PARTIAL;
+  const size_t mark = c.ar.off;
+  float *part = q.part_ext ? q.part_ext
+                           : (partial ? c.ar.take<float>(static_cast<size_t>(splits) * nt * 128 * bn) : nullptr);
+  if (c.dry()) {
+    c.ar.off = mark;
+    return HT_OK;
+  }
+  if (partial && !part) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (gemm scratch)");
+  Gemm3Args g;
+  g.a = q.a3;
+  g.b = q.b3;
+  g.a_plane = q.a3_plane;
+  g.b_plane = q.b3_plane;
+  g.gen = gen;
+  g.splits = splits;
+  g.out_mode = partial ? OUT_PARTIAL : OUT_COLMAJOR;
+  g.out = partial ? part : q.out;
+  g.ld_out = q.ld_out;
+  g.err = c.err;
+  g.a32 = fp32_operand(q.a32);
+  g.b32 = fp32_operand(q.b32);
+  g.guard = c.nf;
+  g.epoch = c.epoch;
+  g.bias = partial ? nullptr : q.bias;
+  g.relu = !partial && q.relu ? 1 : 0;
+  HT_CUDA(tc3_gemm_launch(g, c.st));
+  c.path |= 2;
+  ++c.launches;
+  if (partial && !q.part_ext) {
+    HT_CUDA(reduce_partials_launch(part, gen, splits, bn, q.out, q.ld_out,
+                                   (q.symmetric ? 1 : 0) | (q.accumulate ? 2 : 0), c.st));
+    ++c.launches;
+    if (q.bias || q.relu) {
+      HT_CUDA(bias_act_launch(q.out, q.bias, q.t_n, q.ld_out, q.relu ? 1 : 0, c.st));
+      ++c.launches;
+    }
+  }
+  c.ar.off = mark;
+  return HT_OK;
+}
+
+struct Planes {
+  __nv_bfloat16 *p = nullptr;
+  long long plane = 0;   // elements per plane
+};
+
+// Arena memory for the planes of a rows x cols matrix (rows a multiple of 8).
+ht_status_t reserve_planes(Ctx &c, long long rows, long long cols, Planes *out) {
+  out->plane = (rows * cols + 63) / 64 * 64;
+  out->p = c.ar.take<__nv_bfloat16>(static_cast<size_t>(3 * out->plane));
+  return out->p ? HT_OK : fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (operand planes)");
+}
+
+// Three planes of a rows x cols FP32 matrix (column-major, first index padded
+// to a multiple of 8) in arena memory; *plane = elements per plane.
+ht_status_t take_planes(Ctx &c, const float *x, long long rows, long long cols, __nv_bfloat16 **out, long long *plane,
+                        double *partials = nullptr, int num_partials = 0) {
+  const long long rp = (rows + 7) / 8 * 8;
+  *plane = (rp * cols + 63) / 64 * 64;
+  *out = c.ar.take<__nv_bfloat16>(static_cast<size_t>(3 * *plane));
+  if (!*out) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (operand planes)");
+  if (c.dry()) return HT_OK;
+  HT_CUDA(split3_launch(x, *out, *plane, rows, rp, cols, partials, num_partials, c.nf, c.epoch, c.st));
+  ++c.launches;
   return HT_OK;
 }
 
@@ -469,6 +599,25 @@ ht_status_t gram_padded(Ctx &c, const View &v, const View &vp, const float *x32,
   return run_gemm(c, q);
 }
 
+// The Gram of view v from X's planes, whose view of the same mode group is vp
+// (vp's innermost extent padded to a multiple of 8).
+ht_status_t gram3(Ctx &c, const View &v, const View &vp, const float *x32, const __nv_bfloat16 *x3, long long plane,
+                  float *G) {
+  GemmReq q;
+  q.a32 = q.b32 = gram_operand(v, x32);
+  q.a16.ptr = q.b16.ptr = nullptr;
+  q.a3 = q.b3 = gram_operand(vp, x3);
+  q.a3_plane = q.b3_plane = plane;
+  q.bn_simt = v.N > 64 ? 128 : 64;
+  q.tiles_kind = TILES_GRAM;
+  q.t_n = v.N;
+  q.out_mode = OUT_PARTIAL;
+  q.out = G;
+  q.ld_out = v.N;
+  q.symmetric = true;
+  return run_gemm(c, q);
+}
+
 // l-block exponent of the last mode's second BF16 copy (0: no copy).
 int last_mode_block(const long *dims, int order) {
   if (order != 3) return 0;
@@ -508,8 +657,10 @@ ht_status_t gram_transposed(Ctx &c, const View &v, const float *x32, const __nv_
 // carries W to about 16 significant bits instead of BF16's 8.
 // Z16 non-null: the product is wanted in BF16 there (Z is then FP32 scratch).
 ht_status_t mode_product(Ctx &c, const View &v, const float *x32, const __nv_bfloat16 *x16, const float *W32,
-                         const __nv_bfloat16 *W16, int k, float *Z, int fold_h = 0, __nv_bfloat16 *Z16 = nullptr) {
+                         const __nv_bfloat16 *W16, int k, float *Z, int fold_h = 0, __nv_bfloat16 *Z16 = nullptr,
+                         const View *vp = nullptr, const __nv_bfloat16 *x3 = nullptr, long long x3_plane = 0) {
   GemmReq q;
+  const size_t mark = c.ar.off;
   auto opA = [&](const void *x) {
     Operand o;
     o.ptr = x;
@@ -539,7 +690,22 @@ ht_status_t mode_product(Ctx &c, const View &v, const float *x32, const __nv_bfl
   q.out = Z;
   q.out16 = Z16;
   q.ld_out = v.L * v.R;
-  return run_gemm(c, q);
+  if (x3 && c.tc3) {
+    __nv_bfloat16 *W3 = nullptr;
+    HT_TRY(take_planes(c, W32, v.N, k, &W3, &q.b3_plane));
+    q.a3.ptr = x3;
+    if (v.L == 1) {
+      q.a3.kind = OP_KM3; q.a3.d0 = vp->N; q.a3.d1 = v.R; q.a3.d2 = 1;
+    } else {
+      q.a3.kind = OP_MN3; q.a3.d0 = vp->L; q.a3.d1 = v.N; q.a3.d2 = v.R;
+    }
+    q.a3_plane = x3_plane;
+    q.b3 = opB(W3, k);
+    q.b3.d0 = (v.N + 7) / 8 * 8;
+  }
+  const ht_status_t st = run_gemm(c, q);
+  c.ar.off = mark;   // W's planes: stream-ordered like the GEMM's own scratch
+  return st;
 }
 
 // Z (v.N x k, column-major) = X_(group) Q with Q ((L*R) x k): contract every index but the middle one
@@ -1014,7 +1180,11 @@ ht_status_t decompose_core(Ctx &c, const Tree &T, const ht_config_t &cfg, const 
     for (int m = 0; m < order; ++m) {
       if (G_pre && G_pre[m]) continue;
       const View v = view_of_group(dims, order, m, m);
-      if (x16p) HT_TRY(gram_padded(c, v, view_of_group(pdims, order, m, m), x32, x16p, G[m]));
+      if (c.x3) {
+        long p3[HT_MAX_ORDER];
+        for (int j = 0; j < order; ++j) p3[j] = j == 0 ? c.x3_n1p : dims[j];
+        HT_TRY(gram3(c, v, view_of_group(p3, order, m, m), x32, c.x3, c.x3_plane, G[m]));
+      } else if (x16p) HT_TRY(gram_padded(c, v, view_of_group(pdims, order, m, m), x32, x16p, G[m]));
       else if (m == order - 1 && x16t) HT_TRY(gram_transposed(c, v, x32, x16t, lb, G[m]));
       else HT_TRY(gram(c, v, x32, x16, G[m]));
     }
@@ -1056,7 +1226,12 @@ ht_status_t decompose_core(Ctx &c, const Tree &T, const ht_config_t &cfg, const 
       HT_CUDA(split_bf16_launch(ec.U, dims[P.mc], kz, fold_h, V16, c.st));
       ++c.launches;
     }
-    HT_TRY(mode_product(c, vc, x32, x16, ec.U, V16, kz, Z, fold_h));
+    // X's planes serve the product where their rows are Z's rows: mode 2's rows
+    // (l over modes 0 and 1) are not when the first mode is padded
+    long p3[3] = {c.x3_n1p, dims[1], dims[2]};
+    const View vp3 = view_of_group(p3, 3, P.mc, P.mc);
+    const bool with3 = c.x3 && (P.mc == 0 || c.x3_n1p == dims[0] || (P.mc == 1 && dims[0] > 1));
+    HT_TRY(mode_product(c, vc, x32, x16, ec.U, V16, kz, Z, fold_h, nullptr, &vp3, with3 ? c.x3 : nullptr, c.x3_plane));
     if (sketch && !c.dry()) HT_CUDA(tsqr_launch(Z, zrows, kz, zrows, Rz, tr.WG, qws, qbytes, c.st, &c.launches));
     tl.mark(c.st);
     HT_TRY(transfer3_from_z(c, P, dims, ep, Z, tr, res, sketch));
@@ -1142,6 +1317,116 @@ ht_status_t decompose_core(Ctx &c, const Tree &T, const ht_config_t &cfg, const 
   return HT_OK;
 }
 
+// Slab z of a batch: C_z (m x n, ldc, sC apart) = A_z B^T, A_z = A + z sA (m x k,
+// lda), B n x k (dense), column-major.
+struct NtProduct {
+  const float *A;
+  long long lda, sA;
+  const float *B;
+  const float *C;   // written, or (nt_sqdiff) the matrix compared with
+  long long ldc, sC, m, n;
+  int k;
+  long long batch;
+};
+
+// From these many multiply-adds the products of an HT expansion and the error
+// pass run from operand planes on tcgen05.  Below, the planes' launches (two of
+// ~3 us) and the persistent kernel's start (~5 us) cost more than the CUDA-core
+// kernels: gemm_nt_kernel does ~16 multiply-adds a ns, error_fused_kernel ~5.
+constexpr double kNt3MinMac = 2e8, kSq3MinMac = 5e7;
+
+bool nt_with_planes(const Ctx &c, const NtProduct &p, double min_mac) {
+  const bool dense = p.lda == p.m && (p.batch == 1 || p.sA == p.m * p.k);
+  const bool inner = p.batch > 1 && p.lda == p.m * p.batch && p.sA == p.m;   // slabs between rows and k
+  return c.tc3 && p.k <= 64 && p.batch <= 65535 && (dense || inner) && p.m < (1ll << 31) - 256 &&
+         p.n < (1ll << 31) - 256 && double(p.m) * p.n * p.k * p.batch >= min_mac &&
+         ((p.m + 127) / 128) * ((p.n + 63) / 64) * p.batch < (1ll << 30);
+}
+
+// Operands of a product from planes (arena memory).
+ht_status_t nt_operands(Ctx &c, const NtProduct &p, Gemm3Args *g) {
+  const long long mp = (p.m + 7) / 8 * 8, np = (p.n + 7) / 8 * 8;
+  __nv_bfloat16 *a3 = nullptr, *b3 = nullptr;
+  HT_TRY(take_planes(c, p.A, p.m, static_cast<long long>(p.k) * p.batch, &a3, &g->a_plane));
+  HT_TRY(take_planes(c, p.B, p.n, p.k, &b3, &g->b_plane));
+  g->a.kind = g->b.kind = OP_MN3;
+  g->a.ptr = a3;
+  g->a.d0 = static_cast<long>(mp);
+  g->a.d1 = p.k;
+  g->a.d2 = static_cast<long>(p.batch);
+  if (p.batch > 1 && p.sA == p.m) {
+    g->a.s1 = static_cast<long>(mp * p.batch);
+    g->a.s2 = static_cast<long>(mp);
+  }
+  g->b.ptr = b3;
+  g->b.d0 = static_cast<long>(np);
+  g->b.d1 = p.k;
+  g->b.d2 = 1;
+  if (!make_grid_gen(p.m, p.n, p.n > 128 ? 256 : (p.n > 64 ? 128 : 64), &g->gen, p.batch, p.sC))
+    return fail(HT_ERR_UNSUPPORTED, "product too large for one grid");
+  g->splits = 1;
+  g->out = const_cast<float *>(p.C);
+  g->ld_out = p.ldc;
+  g->err = c.err;
+  g->a32.p = p.A;
+  g->a32.rs = 1; g->a32.ls = p.lda; g->a32.zs = p.sA; g->a32.len = p.k;
+  g->b32.p = p.B;
+  g->b32.rs = 1; g->b32.ls = p.n; g->b32.len = p.k;
+  g->guard = c.nf;
+  g->epoch = c.epoch;
+  return HT_OK;
+}
+
+ht_status_t nt_product(Ctx &c, const NtProduct &p) {
+  const size_t mark = c.ar.off;
+  const bool planes = nt_with_planes(c, p, kNt3MinMac);
+  if (planes) {
+    Gemm3Args g;
+    HT_TRY(nt_operands(c, p, &g));
+    g.out_mode = OUT_COLMAJOR;
+    if (!c.dry()) HT_CUDA(tc3_gemm_launch(g, c.st));
+  }
+  if (!c.dry() && !planes)
+    HT_CUDA(gemm_nt_launch(p.A, p.lda, p.sA, p.B, p.n, const_cast<float *>(p.C), p.ldc, p.sC, p.m, p.n, p.k, p.batch,
+                           c.st));
+  if (!c.dry()) ++c.launches;
+  c.ar.off = mark;
+  return HT_OK;
+}
+
+// sum over z of ||C_z - A_z B^T||^2 as *nparts partial sums in parts.
+ht_status_t nt_sqdiff(Ctx &c, const NtProduct &p, double *parts, int *nparts) {
+  const size_t mark = c.ar.off;
+  if (nt_with_planes(c, p, kSq3MinMac)) {
+    Gemm3Args g;
+    HT_TRY(nt_operands(c, p, &g));
+    g.out_mode = OUT_SQDIFF;
+    g.parts = parts;
+    *nparts = tc3_sq_parts(g);
+    if (!c.dry()) HT_CUDA(tc3_gemm_launch(g, c.st));
+  } else {
+    *nparts = error_fused_blocks(p.m, p.n) * static_cast<int>(p.batch);
+    if (!c.dry())
+      HT_CUDA(error_fused_launch(p.C, p.ldc, p.sC, p.A, p.lda, p.sA, p.B, p.n, p.m, p.n, p.k, static_cast<int>(p.batch),
+                                 parts, c.st));
+  }
+  if (!c.dry()) ++c.launches;
+  c.ar.off = mark;
+  return HT_OK;
+}
+
+// W[i0 + n0*i1 + n0*n1*c] = sum_{a,b} U0[i0,a] U1[i1,b] core[a + k0*b + k0*k1*c]  (T: n0*k1*k2 scratch)
+ht_status_t expand2(Ctx &c, const float *U0, long n0, int k0, const float *core, const float *U1, long n1, int k1, int k2,
+                    float *T, float *W) {
+  if (!c.dry()) {
+    HT_CUDA(expand1_launch(U0, static_cast<int>(n0), k0, core, k1, k2, T, c.st));
+    ++c.launches;
+  }
+  // (ranks are at most 64: parse_tree)
+  return nt_product(c, NtProduct{T, n0, static_cast<long long>(n0) * k1, U1, W, n0, static_cast<long long>(n0) * n1, n0,
+                                 n1, k1, k2});
+}
+
 // ||X - Xhat||_F^2 of an HT representation, into *dev_out (device double).
 ht_status_t error_core(Ctx &c, const Tree &T, const float *x32, const long *dims, int order, const float *const *U,
                        const float *const *B, double *dev_out) {
@@ -1161,7 +1446,7 @@ ht_status_t error_core(Ctx &c, const Tree &T, const float *x32, const long *dims
     else if (P.mc == 0) { Rr = nc_; Cc = np_ * nq_; }
     else { Rr = np_; Cc = nc_; batch = static_cast<int>(nq_); }
     nb = error_fused_blocks(Rr, Cc) * batch;
-    parts = c.ar.take<double>(static_cast<size_t>(nb) + 8);
+    parts = c.ar.take<double>(static_cast<size_t>(std::max(nb, sm_count())) + 8);
     if (!Bkt || !core || !Tm || !Wm || !parts) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (error)");
     c.stage = 4;
     if (c.err_out && !c.ar.dry) {   // the batch's grouped error pass
@@ -1206,17 +1491,19 @@ ht_status_t error_core(Ctx &c, const Tree &T, const float *x32, const long *dims
       else HT_CUDA(transpose_small_launch(B[0], P.kc, P.kt, Bkt, c.st));
       const long long kpq = static_cast<long long>(P.kp) * P.kq;
       HT_CUDA(matmul_nn_launch(B[P.t], kpq, Bkt, P.kt, core, kpq, kpq, P.kc, P.kt, c.st));
-      HT_CUDA(expand2_launch(U[P.p], static_cast<int>(np_), P.kp, core, U[P.q], static_cast<int>(nq_), P.kq, P.kc, Tm,
-                             Wm, c.st));
-      if (P.mc == 2)         // X_(01) = W U_c^T
-        HT_CUDA(error_fused_launch(x32, Rr, 0, Wm, Rr, 0, U[P.c], nc_, Rr, Cc, P.kc, 1, parts, c.st));
-      else if (P.mc == 0)    // X_(0) = U_c W^T
-        HT_CUDA(error_fused_launch(x32, Rr, 0, U[P.c], nc_, 0, Wm, np_ * nq_, Rr, Cc, P.kc, 1, parts, c.st));
-      else                   // slab i2 of X (n0 x n1) = W[(i0, i2), :] U_1^T
-        HT_CUDA(error_fused_launch(x32, np_, np_ * nc_, Wm, np_ * nq_, np_, U[P.c], nc_, Rr, Cc, P.kc, batch, parts,
-                                   c.st));
-      c.launches += 5;
+      c.launches += 2;
     }
+    HT_TRY(expand2(c, U[P.p], np_, P.kp, core, U[P.q], nq_, P.kq, P.kc, Tm, Wm));
+    NtProduct e{};
+    e.C = x32; e.m = Rr; e.n = Cc; e.k = P.kc; e.batch = batch; e.ldc = Rr; e.lda = Rr;
+    if (P.mc == 2) {           // X_(01) = W U_c^T
+      e.A = Wm; e.B = U[P.c];
+    } else if (P.mc == 0) {    // X_(0) = U_c W^T
+      e.A = U[P.c]; e.B = Wm;
+    } else {                   // slab i2 of X (n0 x n1) = W[(i0, i2), :] U_1^T
+      e.A = Wm; e.lda = np_ * nq_; e.sA = np_; e.B = U[P.c]; e.sC = np_ * nc_;
+    }
+    HT_TRY(nt_sqdiff(c, e, parts, &nb));
   } else {
     const int t1 = T.left[0], t2 = T.right[0];
     const int k1 = T.rank[t1], k2 = T.rank[t2];
@@ -1228,17 +1515,17 @@ ht_status_t error_core(Ctx &c, const Tree &T, const float *x32, const long *dims
     float *T2 = c.ar.take<float>(static_cast<size_t>(dims[2]) * T.rank[b2] * k2);
     float *W34 = c.ar.take<float>(static_cast<size_t>(Cn) * k2);
     nb = error_fused_blocks(R, Cn);
-    parts = c.ar.take<double>(static_cast<size_t>(nb) + 8);
+    parts = c.ar.take<double>(static_cast<size_t>(std::max(nb, sm_count())) + 8);
     if (!T1 || !W12 || !A12 || !T2 || !W34 || !parts) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (error)");
+    HT_TRY(expand2(c, U[a1], dims[0], T.rank[a1], B[t1], U[b1], dims[1], T.rank[b1], k1, T1, W12));
+    HT_TRY(expand2(c, U[a2], dims[2], T.rank[a2], B[t2], U[b2], dims[3], T.rank[b2], k2, T2, W34));
     if (!c.dry()) {
-      HT_CUDA(expand2_launch(U[a1], static_cast<int>(dims[0]), T.rank[a1], B[t1], U[b1], static_cast<int>(dims[1]),
-                             T.rank[b1], k1, T1, W12, c.st));
-      HT_CUDA(expand2_launch(U[a2], static_cast<int>(dims[2]), T.rank[a2], B[t2], U[b2], static_cast<int>(dims[3]),
-                             T.rank[b2], k2, T2, W34, c.st));
       HT_CUDA(matmul_nn_launch(W12, R, B[0], k1, A12, R, R, k2, k1, c.st));
-      HT_CUDA(error_fused_launch(x32, R, 0, A12, R, 0, W34, Cn, R, Cn, k2, 1, parts, c.st));
-      c.launches += 6;
+      ++c.launches;
     }
+    NtProduct e{};
+    e.C = x32; e.m = R; e.n = Cn; e.k = k2; e.batch = 1; e.ldc = R; e.A = A12; e.lda = R; e.B = W34;
+    HT_TRY(nt_sqdiff(c, e, parts, &nb));
   }
   if (!c.dry()) {   // (stage 4 for 3rd order: part of the grouped error pass)
     HT_CUDA(sumsq_finish_launch(parts, nb, dev_out, c.st));
@@ -1477,10 +1764,9 @@ ht_status_t stream_call(Ctx &c, const Tree &T, const ht_config_t &cfg, const Str
       else HT_CUDA(transpose_small_launch(res.B[0], P.kc, P.kt, Bkt, c.st));
       const long long kpq = static_cast<long long>(P.kp) * P.kq;
       HT_CUDA(matmul_nn_launch(res.B[P.t], kpq, Bkt, P.kt, core, kpq, kpq, P.kc, P.kt, c.st));
-      HT_CUDA(expand2_launch(res.U[P.p], static_cast<int>(np_), P.kp, core, res.U[P.q], static_cast<int>(nq_), P.kq,
-                             P.kc, Tm, Wm, c.st));
-      c.launches += 4;
+      c.launches += 2;
     }
+    HT_TRY(expand2(c, res.U[P.p], np_, P.kp, core, res.U[P.q], nq_, P.kq, P.kc, Tm, Wm));
     HT_TRY(stream_slabs(c, io, cnt2, copy2, [&](long long s, const float *x) -> ht_status_t {
       if (c.dry()) return HT_OK;
       const long long c0 = s * s2, len = std::min(s2, n2 - c0);
@@ -1570,6 +1856,12 @@ ht_status_t enqueue_body(Ctx &c, const Tree &T, const ht_config_t &cfg, const fl
     } else if (!c.dry()) {
       HT_CUDA(convert_bf16_launch(xd, xb, total, nparts, 1024, c.st));
     }
+  } else if (c.tc3 && cfg.leaf_method == HT_LEAF_GRAM) {   // FP32 path: 6 bytes an entry
+    __nv_bfloat16 *planes = nullptr;
+    HT_TRY(take_planes(c, xd, n1, total / n1, &planes, &c.x3_plane, nparts, 1024));
+    c.launches -= c.dry() ? 0 : 1;   // counted with the sums below
+    c.x3 = planes;
+    c.x3_n1p = n1p;
   } else if (!c.dry()) {
     HT_CUDA(sumsq_launch(xd, total, nparts, 1024, c.st));
   }
@@ -1838,9 +2130,10 @@ ht_status_t run_call(Ctx &c, const Tree &T, const ht_config_t &cfg, const CallAr
   return HT_OK;
 }
 
-size_t dry_run_bytes(const Tree &T, const ht_config_t &cfg, const CallArgs &a, int eig_mode = 0) {
+size_t dry_run_bytes(const Tree &T, const ht_config_t &cfg, const CallArgs &a, int eig_mode = 0, bool tc3 = false) {
   Ctx d;
   d.ar.dry = true;
+  d.tc3 = tc3;
   d.eig_mode = eig_mode;
   d.tc = cfg.precision == HT_PREC_BF16;
   run_call(d, T, cfg, a, nullptr);
@@ -2268,7 +2561,8 @@ ht_status_t ht_workspace_size(const long *dims, int order, const ht_tree_t *tree
   ht_config_default(&def);
   float *none[HT_MAX_NODES] = {};
   CallArgs a{nullptr, true, dims, order, none, none, cfg ? (cfg->flags & HT_FLAG_COMPUTE_ERROR) != 0 : false};
-  *bytes = dry_run_bytes(T, cfg ? *cfg : def, a);
+  const ht_config_t &used = cfg ? *cfg : def;
+  *bytes = dry_run_bytes(T, used, a, 0, true);
   return HT_OK;
 }
 
@@ -2293,7 +2587,7 @@ ht_status_t ht_release_workspace(void) {
 // dry run's plan depends on: the device, the dims, the tree, the configuration
 // (its sketch blocks as absent / host / device), where X lives and its 16-byte
 // alignment, and whether the error pass runs.  Call with g_ws_mutex held.
-ht_status_t sized_call_bytes(const Tree &T, const ht_config_t &cfg, const CallArgs &a, size_t *bytes) {
+ht_status_t sized_call_bytes(const Tree &T, const ht_config_t &cfg, const CallArgs &a, bool tc3, size_t *bytes) {
   int dev = 0;
   HT_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(HT_ERR_INVALID_ARG, "device index out of range");
@@ -2316,6 +2610,7 @@ ht_status_t sized_call_bytes(const Tree &T, const ht_config_t &cfg, const CallAr
   key[n++] = a.x_dev;
   key[n++] = static_cast<long long>(reinterpret_cast<uintptr_t>(a.x) & 15u);
   key[n++] = a.want_err;
+  key[n++] = tc3;
   const std::string k(reinterpret_cast<const char *>(key), sizeof(long long) * n);
   auto &cache = g_call[dev].sizes;
   for (const auto &e : cache)
@@ -2323,7 +2618,7 @@ ht_status_t sized_call_bytes(const Tree &T, const ht_config_t &cfg, const CallAr
       *bytes = e.second;
       return HT_OK;
     }
-  *bytes = dry_run_bytes(T, cfg, a);
+  *bytes = dry_run_bytes(T, cfg, a, 0, tc3);
   if (cache.size() >= 64) cache.erase(cache.begin());
   cache.emplace_back(k, *bytes);
   return HT_OK;
@@ -2349,12 +2644,21 @@ ht_status_t ht_decompose(const float *x, const long *dims, int order, const ht_t
   std::lock_guard<std::mutex> lk(g_ws_mutex);
   CallArgs a{x, is_device_ptr(x), dims, order, U, B, (cfg.flags & HT_FLAG_COMPUTE_ERROR) != 0};
   size_t bytes = 0;
-  HT_TRY(sized_call_bytes(T, cfg, a, &bytes));
+  bool tc3 = true;   // FP32 products from operand planes (Ctx::tc3)
+  HT_TRY(sized_call_bytes(T, cfg, a, tc3, &bytes));
   void *ws = nullptr;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  HT_TRY(acquire_workspace(bytes, &ws, st));
+  ht_status_t got = acquire_workspace(bytes, &ws, st);
+  if (got == HT_ERR_OUT_OF_MEMORY && tc3) {   // no room for the planes: CUDA cores
+    cudaGetLastError();
+    tc3 = false;
+    HT_TRY(sized_call_bytes(T, cfg, a, tc3, &bytes));
+    got = acquire_workspace(bytes, &ws, st);
+  }
+  HT_TRY(got);
   Ctx c;
   c.st = st;
+  c.tc3 = tc3;
   c.tc = cfg.precision == HT_PREC_BF16;
   c.ar.base = static_cast<char *>(ws);
   c.ar.cap = bytes;
@@ -2871,16 +3175,20 @@ static ht_status_t reconstruct_core(Ctx &c, const Tree &T, const long *dims, int
       else HT_CUDA(transpose_small_launch(B[0], P.kc, P.kt, Bkt, c.st));
       const long long kpq = static_cast<long long>(P.kp) * P.kq;
       HT_CUDA(matmul_nn_launch(B[P.t], kpq, Bkt, P.kt, core, kpq, kpq, P.kc, P.kt, c.st));
-      HT_CUDA(expand2_launch(U[P.p], static_cast<int>(np_), P.kp, core, U[P.q], static_cast<int>(nq_), P.kq, P.kc, Tm,
-                             Wm, c.st));
-      if (P.mc == 2)        // X_(01) = W U_2^T
-        HT_CUDA(gemm_nt_launch(Wm, np_ * nq_, 0, U[P.c], nc_, out, np_ * nq_, 0, np_ * nq_, nc_, P.kc, 1, c.st));
-      else if (P.mc == 0)   // X_(0) = U_0 W^T
-        HT_CUDA(gemm_nt_launch(U[P.c], nc_, 0, Wm, np_ * nq_, out, nc_, 0, nc_, np_ * nq_, P.kc, 1, c.st));
-      else                  // slab i2: X(:, :, i2) = W[(:, i2), :] U_1^T
-        HT_CUDA(gemm_nt_launch(Wm, np_ * nq_, np_, U[P.c], nc_, out, np_, np_ * nc_, np_, nc_, P.kc, nq_, c.st));
-      c.launches += 4;
+      c.launches += 2;
     }
+    HT_TRY(expand2(c, U[P.p], np_, P.kp, core, U[P.q], nq_, P.kq, P.kc, Tm, Wm));
+    NtProduct e{};
+    e.C = out; e.k = P.kc; e.batch = 1;
+    if (P.mc == 2) {          // X_(01) = W U_2^T
+      e.A = Wm; e.B = U[P.c]; e.m = np_ * nq_; e.n = nc_; e.lda = e.ldc = e.m;
+    } else if (P.mc == 0) {   // X_(0) = U_0 W^T
+      e.A = U[P.c]; e.B = Wm; e.m = nc_; e.n = np_ * nq_; e.lda = e.ldc = e.m;
+    } else {                  // slab i2: X(:, :, i2) = W[(:, i2), :] U_1^T
+      e.A = Wm; e.B = U[P.c]; e.m = e.ldc = np_; e.n = nc_; e.lda = np_ * nq_; e.sA = np_; e.sC = np_ * nc_;
+      e.batch = nq_;
+    }
+    HT_TRY(nt_product(c, e));
   } else {
     const int t1 = T.left[0], t2 = T.right[0];
     const int k1 = T.rank[t1], k2 = T.rank[t2];
@@ -2892,15 +3200,13 @@ static ht_status_t reconstruct_core(Ctx &c, const Tree &T, const long *dims, int
     float *T2 = c.ar.take<float>(static_cast<size_t>(dims[2]) * T.rank[b2] * k2);
     float *W34 = c.ar.take<float>(static_cast<size_t>(Cn) * k2);
     if (!T1 || !W12 || !A12 || !T2 || !W34) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (reconstruct)");
+    HT_TRY(expand2(c, U[a1], dims[0], T.rank[a1], B[t1], U[b1], dims[1], T.rank[b1], k1, T1, W12));
+    HT_TRY(expand2(c, U[a2], dims[2], T.rank[a2], B[t2], U[b2], dims[3], T.rank[b2], k2, T2, W34));
     if (!c.dry()) {
-      HT_CUDA(expand2_launch(U[a1], static_cast<int>(dims[0]), T.rank[a1], B[t1], U[b1], static_cast<int>(dims[1]),
-                             T.rank[b1], k1, T1, W12, c.st));
-      HT_CUDA(expand2_launch(U[a2], static_cast<int>(dims[2]), T.rank[a2], B[t2], U[b2], static_cast<int>(dims[3]),
-                             T.rank[b2], k2, T2, W34, c.st));
       HT_CUDA(matmul_nn_launch(W12, R, B[0], k1, A12, R, R, k2, k1, c.st));
-      HT_CUDA(gemm_nt_launch(A12, R, 0, W34, Cn, out, R, 0, R, Cn, k2, 1, c.st));
-      c.launches += 6;
+      ++c.launches;
     }
+    HT_TRY(nt_product(c, NtProduct{A12, R, 0, W34, out, R, 0, R, Cn, k2, 1}));
   }
   c.ar.off = mark;
   return HT_OK;
@@ -2921,6 +3227,11 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto plan = [&](Ctx &c) -> ht_status_t {
     const float *Ud[HT_MAX_NODES] = {}, *Bd[HT_MAX_NODES] = {};
+    c.err = c.ar.take<int>(64);
+    if (!c.err) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small");
+    c.nf = c.err + 32;
+    c.epoch = 1;
+    if (!c.dry()) HT_CUDA(cudaMemsetAsync(c.err, 0, 64 * sizeof(int), c.st));
     HT_TRY(stage_factors(c, T, dims, U, B, Ud, Bd));
     float *o = out_dev ? x_out : c.ar.take<float>(static_cast<size_t>(total));
     if (!o) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small");
@@ -2929,18 +3240,34 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
       HT_CUDA(cudaMemcpyAsync(x_out, o, sizeof(float) * total, cudaMemcpyDeviceToHost, c.st));
     return HT_OK;
   };
-  Ctx d;
-  d.ar.dry = true;
-  HT_TRY(plan(d));
-  const size_t bytes = d.ar.peak + (1 << 20);
   void *ws = nullptr;
-  HT_TRY(acquire_workspace(bytes, &ws, st));
+  size_t bytes = 0;
+  bool tc3 = true;
+  auto acquire = [&]() -> ht_status_t {
+    Ctx d;
+    d.ar.dry = true;
+    d.tc3 = tc3;
+    HT_TRY(plan(d));
+    bytes = d.ar.peak + (1 << 20);
+    return acquire_workspace(bytes, &ws, st);
+  };
+  ht_status_t got = acquire();
+  if (got == HT_ERR_OUT_OF_MEMORY) {   // no room for the planes: CUDA cores
+    cudaGetLastError();
+    tc3 = false;
+    got = acquire();
+  }
+  HT_TRY(got);
   Ctx c;
   c.st = st;
+  c.tc3 = tc3;
   c.ar.base = static_cast<char *>(ws);
   c.ar.cap = bytes;
   HT_TRY(plan(c));
+  int errword = 0;
+  HT_CUDA(cudaMemcpyAsync(&errword, c.err, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   HT_CUDA(cudaStreamSynchronize(c.st));
+  if (errword & kErrTimeout) return fail(HT_ERR_TIMEOUT, "a kernel's bounded wait expired; results are invalid");
   g_launches += static_cast<unsigned long long>(c.launches);
   return HT_OK;
 }
@@ -3420,6 +3747,7 @@ namespace {
 
 std::mutex g_layer_mutex;
 DeviceWorkspace g_layer_ws[64];
+int g_layer_epoch[64];  // calls since the workspace was made (Ctx::epoch)
 int *g_layer_err[64];   // first 256 bytes of each device's layer workspace
 
 ht_status_t layer_shape(const ht_layer_shape_t *in, LayerShape *sh) {
@@ -3468,11 +3796,18 @@ ht_status_t layer_run(cudaStream_t st, bool tc, F &&plan) {
   int dev = 0;
   HT_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(HT_ERR_INVALID_ARG, "device index out of range");
-  Ctx d;
-  d.ar.dry = true;
-  d.tc = tc;
-  HT_TRY(plan(d));
-  const size_t bytes = d.ar.peak + 256 + (1 << 16);
+  bool tc3 = !tc;
+  size_t bytes = 0;
+  auto size = [&]() -> ht_status_t {
+    Ctx d;
+    d.ar.dry = true;
+    d.tc = tc;
+    d.tc3 = tc3;
+    HT_TRY(plan(d));
+    bytes = d.ar.peak + 256 + (1 << 16);
+    return HT_OK;
+  };
+  HT_TRY(size());
   std::lock_guard<std::mutex> lk(g_layer_mutex);
   DeviceWorkspace &w = g_layer_ws[dev];
   if (w.bytes < bytes) {
@@ -3482,16 +3817,27 @@ ht_status_t layer_run(cudaStream_t st, bool tc, F &&plan) {
       w.ptr = nullptr;
       w.bytes = 0;
     }
-    HT_CUDA(cudaMalloc(&w.ptr, bytes));
+    cudaError_t e = cudaMalloc(&w.ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && tc3) {   // no room for the operands' planes: CUDA cores
+      cudaGetLastError();
+      tc3 = false;
+      HT_TRY(size());
+      e = cudaMalloc(&w.ptr, bytes);
+    }
+    HT_CUDA(e);
     HT_CUDA(cudaMemset(w.ptr, 0, 256));
     HT_CUDA(cudaDeviceSynchronize());
     w.bytes = bytes;
     g_layer_err[dev] = static_cast<int *>(w.ptr);
+    g_layer_epoch[dev] = 0;
   }
   Ctx c;
   c.st = st;
   c.tc = tc;
+  c.tc3 = tc3;
   c.err = g_layer_err[dev];
+  c.nf = g_layer_err[dev] + 32;   // its own 128 bytes behind the error word
+  c.epoch = ++g_layer_epoch[dev];
   c.ar.base = static_cast<char *>(w.ptr) + 256;
   c.ar.cap = w.bytes - 256;
   HT_TRY(plan(c));
@@ -3500,11 +3846,21 @@ ht_status_t layer_run(cudaStream_t st, bool tc, F &&plan) {
 }
 
 // D (rows x cols, column-major, ld = rows) = A B^T over the two operand pairs.
+// a3 / b3: the FP32 operands' planes (ptr null: none, the CUDA cores form the product).
 ht_status_t layer_gemm(Ctx &c, const Operand &a32, const Operand &b32, const Operand &a16, const Operand &b16,
-                       long long rows, long long cols, float *D) {
+                       const Planes &a3, const Planes &b3, long long rows, long long cols, float *D,
+                       const float *bias = nullptr, bool relu = false) {
   GemmReq q;
   q.a32 = a32;
   q.b32 = b32;
+  q.a3 = a32;
+  q.b3 = b32;
+  q.a3.ptr = a3.p;
+  q.b3.ptr = b3.p;
+  q.a3_plane = a3.plane;
+  q.b3_plane = b3.plane;
+  q.bias = bias;
+  q.relu = relu;
   q.a16 = a16;
   q.b16 = b16;
   q.bn_tc = cols >= 256 ? 256 : (cols > 64 ? 128 : 64);
@@ -3555,7 +3911,7 @@ ht_status_t ht_layer_weight(const ht_layer_shape_t *shape, const float *u1, cons
     if (!P || !Q) return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
     if (c.dry()) return HT_OK;
     HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st));
-    HT_CUDA(layer_weight_launch(sh, P, Q, W, nullptr, c.st));
+    HT_CUDA(layer_weight_launch(sh, P, Q, W, nullptr, nullptr, 0, nullptr, 0, c.st));
     c.launches += 2;
     return HT_OK;
   });
@@ -3583,20 +3939,20 @@ ht_status_t ht_layer_forward(const ht_layer_shape_t *shape, const float *u1, con
     float *W32 = tc ? nullptr : c.ar.take<float>(static_cast<size_t>(nin * nout));
     __nv_bfloat16 *W16 = tc ? c.ar.take<__nv_bfloat16>(static_cast<size_t>(nin * nout)) : nullptr;
     __nv_bfloat16 *x16 = tc ? c.ar.take<__nv_bfloat16>(static_cast<size_t>(batch * nin)) : nullptr;
+    Planes W3, x3;
+    if (c.tc3 && nin % 8 == 0) HT_TRY(reserve_planes(c, nin, nout, &W3));
     if (!P || !Q || !(W32 || W16) || (tc && !x16)) return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
     if (!c.dry()) {
       HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st));
-      HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, c.st));
+      HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.epoch, c.st));
       if (tc) HT_CUDA(f32_to_bf16_launch(x, x16, batch * nin, c.st));
       c.launches += tc ? 3 : 2;
     }
+    if (W3.p) HT_TRY(take_planes(c, x, nin, batch, &x3.p, &x3.plane));
     // y^T (nout x batch, column-major) = W x^T: A = W (rows o, K-major), B = x (rows z, K-major)
     HT_TRY(layer_gemm(c, op_of(OP_KM3, W32, nin, nout), op_of(OP_KM3, x, nin, batch),
-                      op_of(OP_KM3, W16, nin, nout), op_of(OP_KM3, x16, nin, batch), nout, batch, y));
-    if (!c.dry() && (bias || activation)) {
-      HT_CUDA(bias_act_launch(y, bias, batch, nout, activation, c.st));
-      ++c.launches;
-    }
+                      op_of(OP_KM3, W16, nin, nout), op_of(OP_KM3, x16, nin, batch), W3, x3, nout, batch, y, bias,
+                      activation == 1));
     return HT_OK;
   });
 }
@@ -3636,11 +3992,17 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
     if (!P || !Q || !T1 || !dP || !dQ || !dT1 || !dW || (dx && !(W32 || W16)) || (tc && (!x16 || !dy16)) ||
         (dbias && !part) || (nqp && !dQpart))
       return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
+    Planes W3, x3, dy3;
+    if (c.tc3 && nin % 8 == 0 && nout % 8 == 0) {
+      if (dx) HT_TRY(reserve_planes(c, nin, nout, &W3));
+      HT_TRY(reserve_planes(c, nin, batch, &x3));
+      HT_TRY(reserve_planes(c, nout, batch, &dy3));
+    }
     if (!c.dry()) {
       HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, T1, c.st));
       ++c.launches;
       if (dx) {
-        HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, c.st));
+        HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.epoch, c.st));
         ++c.launches;
       }
       if (tc) {
@@ -3649,12 +4011,23 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
         c.launches += 2;
       }
     }
+    if (x3.p && !c.dry()) {
+      if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 15u) == 0) {
+        HT_CUDA(split3_pair_launch(x, x3.p, x3.plane, batch * nin, dy, dy3.p, dy3.plane, batch * nout, c.nf, c.epoch,
+                                   c.st));
+        ++c.launches;
+      } else {
+        HT_CUDA(split3_launch(x, x3.p, x3.plane, nin, nin, batch, nullptr, 0, c.nf, c.epoch, c.st));
+        HT_CUDA(split3_launch(dy, dy3.p, dy3.plane, nout, nout, batch, nullptr, 0, c.nf, c.epoch, c.st));
+        c.launches += 2;
+      }
+    }
     if (dx)   // dx^T (nin x batch) = W^T dy^T: A = W^T (rows i, MN-major), B = dy (rows z, K-major)
       HT_TRY(layer_gemm(c, op_of(OP_MN3, W32, nin, nout), op_of(OP_KM3, dy, nout, batch),
-                        op_of(OP_MN3, W16, nin, nout), op_of(OP_KM3, dy16, nout, batch), nin, batch, dx));
+                        op_of(OP_MN3, W16, nin, nout), op_of(OP_KM3, dy16, nout, batch), W3, dy3, nin, batch, dx));
     // dW^T (nin x nout, column-major = dW row-major) = x^T dy: A = x^T (rows i), B = dy^T (rows o), K = z
     HT_TRY(layer_gemm(c, op_of(OP_MN3, x, nin, batch), op_of(OP_MN3, dy, nout, batch),
-                      op_of(OP_MN3, x16, nin, batch), op_of(OP_MN3, dy16, nout, batch), nin, nout, dW));
+                      op_of(OP_MN3, x16, nin, batch), op_of(OP_MN3, dy16, nout, batch), x3, dy3, nin, nout, dW));
     if (!c.dry()) {
       if (dbias) {
         HT_CUDA(layer_colsum_launch(dy, batch, nout, part, dbias, c.st));

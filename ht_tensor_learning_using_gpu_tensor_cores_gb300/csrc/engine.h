@@ -1,6 +1,7 @@
 // Internal interfaces between the host orchestration (api.cu) and the kernel
 // translation units.  Not part of the public C ABI.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -30,6 +31,7 @@ struct Operand {
   int kind;
   const void *ptr;      // __nv_bfloat16* for the tcgen05 path, float* for the SIMT path
   long d0, d1, d2;
+  long s1 = 0, s2 = 0;  // three-plane operands: strides of d1, d2 when not dense
 };
 
 // One output tile.  a_row / b_row: first row of the A / B operand;
@@ -41,7 +43,7 @@ struct Tile {
   int out_col, valid_cols;
 };
 
-enum OutMode : int { OUT_PARTIAL = 0, OUT_COLMAJOR = 1 };
+enum OutMode : int { OUT_PARTIAL = 0, OUT_COLMAJOR = 1, OUT_SQDIFF = 2 };
 
 // Output tiles are generated from a small descriptor passed by value in the
 // kernel parameters (no host->device copy on the launch path).
@@ -49,7 +51,8 @@ enum TileKind : int {
   TILES_ROWS = 0,   // rows [0, rows) in blocks of 128, one column block
   TILES_SLABS = 1,  // (l-block, r) blocks of a (L, *, R) view, out_row = l + L*r
   TILES_GRAM = 2,   // blocks of an n x n symmetric matrix on or above the diagonal
-  TILES_GRID = 3    // bm x bn blocks of a rows x n output, row block fastest
+  TILES_GRID = 3    // bm x bn blocks of a rows x n output, row block fastest; R > 1: R such outputs
+                    // (A's d2 coordinate 0..R-1), L elements apart
 };
 constexpr int kMaxGramRows = 256;   // n <= 32768
 struct TileGen {
@@ -80,6 +83,8 @@ struct GemmArgs {
   // tcgen05 path, column-major output only: non-null = write the output in
   // BF16 here instead of FP32 to `out`
   __nv_bfloat16 *out16 = nullptr;
+  const float *bias = nullptr;   // tcgen05 path, column-major FP32 output: bias of row r added, then ReLU when relu
+  int relu = 0;
 };
 
 // tcgen05 path (BF16 operands), BM = 128, BN in {64, 128, 256}.
@@ -102,6 +107,48 @@ cudaError_t tc_gemm_launch(const GemmArgs &g, int bn, cudaStream_t s);
 cudaError_t tc_prepare();
 // number of 64-wide K blocks of an operand pair (tcgen05 path)
 long tc_num_kblocks(const Operand &a);
+
+// FP32-accurate products on tcgen05 (tc3_gemm.cu): operands as three BF16
+// planes (`plane` elements apart, the first at Operand::ptr), tiles 128 x BN,
+// BN in {64, 128, 256} = gen.bn.
+// FP32 entries of an operand: row, l, r, z (see OpKind) at
+// row * rs + l * ls + r * rr + z * zs; l runs over len before r advances.
+struct Fp32Operand {
+  const float *p = nullptr;
+  long long rs = 0, ls = 0, rr = 0, zs = 0, len = 0;
+};
+struct Gemm3Args {
+  Operand a, b;
+  // non-null guard: *guard == epoch (an operand entry had no planes, see
+  // split3_launch) makes the launch form the product from a32, b32 instead
+  Fp32Operand a32, b32;
+  const int *guard = nullptr;
+  int epoch = 0;
+  long long a_plane, b_plane;
+  TileGen gen;
+  int splits, out_mode;
+  float *out;
+  long long ld_out;
+  int *err;
+  const float *bias = nullptr;   // column-major output: bias of row r added to it
+  int relu = 0;
+  double *parts = nullptr;       // OUT_SQDIFF (splits = 1): tc3_sq_parts(g) sums; out = the compared matrix
+};
+int tc3_sq_parts(const Gemm3Args &g);
+Fp32Operand fp32_operand(const Operand &o);
+bool tc3_supported(const Operand &a, long long a_plane, const Operand &b, long long b_plane);
+cudaError_t tc3_gemm_launch(const Gemm3Args &g, cudaStream_t s);
+long tc3_num_kblocks(const Operand &a);
+// x (n1 x rest) -> three planes of n1p x rest (zero rows n1 <= i < n1p), n1p a
+// multiple of 8; partials non-null: also num_partials block sums of squares;
+// flag non-null: *flag = epoch when an entry has no planes (not finite).
+// A second array (x2, elements in multiples of 8, 16-byte aligned like x) can
+// ride along when x needs no padding and no sums.
+cudaError_t split3_pair_launch(const float *x, __nv_bfloat16 *planes, long long plane, long long n, const float *x2,
+                               __nv_bfloat16 *planes2, long long plane2, long long n2, int *flag, int epoch,
+                               cudaStream_t s);
+cudaError_t split3_launch(const float *x, __nv_bfloat16 *planes, long long plane, long long n1, long long n1p,
+                          long long rest, double *partials, int num_partials, int *flag, int epoch, cudaStream_t s);
 
 // SIMT FP32 path (float operands), BM = 128, BN in {64, 128}.
 // Grouped FP32 GEMMs of the batched path (the 3rd-order core pass): every
@@ -131,7 +178,7 @@ cudaError_t reduce_partials_launch(const float *partial, const TileGen &gen, int
 TileGen make_rows_gen(long long rows, int cols, int bn);
 TileGen make_slabs_gen(long long L, long long R, int cols, int bn);
 // rows x cols output in 128 x bn tiles (TILES_GRID); false when the tile count overflows
-bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g);
+bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long batch = 1, long long zstride = 0);
 bool make_gram_gen(long long n, int bn, TileGen *g, int bm = 128);
 
 // Multiprocessor count of the current device (cached per device).
@@ -249,9 +296,9 @@ cudaError_t gemm_tn_small_launch(const float *A, int lda, const float *B, int ld
 int core_step2_ranges(int nq, int kc);
 cudaError_t core_step2_launch(const float *T1, long long ldt, int nq, int kp, const float *Uq, int kq, int kc, float *C,
                               float *scratch, cudaStream_t s);
-// W[i0 + n0*i1 + n0*n1*c] = sum_{a,b} U0[i0,a] U1[i1,b] core[a + k0*b + k0*k1*c]  (T: n0*k1*k2 scratch)
-cudaError_t expand2_launch(const float *U0, int n0, int k0, const float *core, const float *U1, int n1, int k1, int k2,
-                           float *T, float *W, cudaStream_t s);
+// T[i0 + n0*(b + k1*c)] = sum_a U0[i0,a] core[a + k0*b + k0*k1*c]
+cudaError_t expand1_launch(const float *U0, int n0, int k0, const float *core, int k1, int k2, float *T,
+                           cudaStream_t s);
 // C (m x n) = A (m x K) B (K x n), column-major
 cudaError_t matmul_nn_launch(const float *A, long long lda, const float *B, int ldb, float *C, long long ldc,
                              long long m, int n, int K, cudaStream_t s);
@@ -401,7 +448,7 @@ cudaError_t layer_pq_launch(const LayerShape &sh, const float *u1, const float *
                             const float *b1, float *P, float *Q, float *T1, cudaStream_t s);
 // W (Nout x Nin, row-major) from P and Q, into W32 (FP32) or, when W32 is null, W16 (BF16)
 cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
-                                cudaStream_t s);
+                                __nv_bfloat16 *W3, long long plane, int *flag, int epoch, cudaStream_t s);
 // y[z, o] = act(y[z, o] + bias[o]) (bias may be null; act 0 identity, 1 ReLU)
 cudaError_t bias_act_launch(float *y, const float *bias, long long batch, long long nout, int act, cudaStream_t s);
 // out[o] = sum_z dy[z, o]; part holds layer_colsum_chunks(batch) * nout floats

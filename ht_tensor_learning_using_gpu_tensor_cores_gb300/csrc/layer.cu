@@ -69,18 +69,36 @@ __global__ void __launch_bounds__(kLayerThreads) layer_pq_kernel(const LayerShap
   }
 }
 
-template <class T>
-HT_DEV T from_f32(float v);
-template <>
-HT_DEV float from_f32<float>(float v) { return v; }
-template <>
-HT_DEV __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+// Where a weight goes: FP32, BF16, or the three BF16 planes of an FP32-accurate
+// product (tc3_gemm.cu), the FP32 weight beside them.
+struct WeightOut {
+  float *w32;
+  __nv_bfloat16 *w16, *w3;
+  long long plane;
+};
+enum WeightKind : int { W_FP32 = 0, W_BF16 = 1, W_PLANES = 2 };
+template <int KIND>
+HT_DEV void put_weight(const WeightOut &W, long long e, float v) {
+  if (KIND != W_BF16) W.w32[e] = v;
+  if (KIND == W_BF16) W.w16[e] = __float2bfloat16_rn(v);
+  if (KIND == W_PLANES) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    const float r = v - __bfloat162float(h);
+    const __nv_bfloat16 m = __float2bfloat16_rn(r);
+    W.w3[e] = h;
+    W.w3[W.plane + e] = m;
+    W.w3[2 * W.plane + e] = __float2bfloat16_rn(r - __bfloat162float(m));
+  }
+}
+// An entry without planes (not finite once rounded to BF16): see split3_launch.
+HT_DEV bool no_planes(float v) { return !(fabsf(__bfloat162float(__float2bfloat16_rn(v))) <= 3.4e38f); }
 
 // W[o * Nin + i] = sum_r1 P[a, b, r1] Q[c, r1]; i = (n0 N1 + n1) N2 + n2 runs
 // fastest, so consecutive threads share (a, b) and read P's row once.
-template <class T>
+template <int KIND>
 __global__ void __launch_bounds__(kLayerThreads) layer_weight_kernel(const LayerShape sh, const float *__restrict__ P,
-                                                                     const float *__restrict__ Q, T *__restrict__ W) {
+                                                                     const float *__restrict__ Q, const WeightOut W,
+                                                                     int *flag, int epoch) {
   const int N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
   const long long Nin = static_cast<long long>(sh.n[0]) * N1 * N2, Nout = static_cast<long long>(M0) * M1 * M2;
   const int B = N1 * M1, R1 = sh.r1;
@@ -94,7 +112,8 @@ __global__ void __launch_bounds__(kLayerThreads) layer_weight_kernel(const Layer
     const float *q = Q + static_cast<long long>(c) * R1;
     float s = 0.f;
     for (int r = 0; r < R1; ++r) s = fmaf(p[r], q[r], s);
-    W[e] = from_f32<T>(s);
+    put_weight<KIND>(W, e, s);
+    if (KIND == W_PLANES && no_planes(s)) *flag = epoch;
   }
 }
 
@@ -104,11 +123,11 @@ __global__ void __launch_bounds__(kLayerThreads) layer_weight_kernel(const Layer
 // accumulators for one input index i and writes kWeightG rows of W, consecutive
 // threads on consecutive i (coalesced rows).
 constexpr int kWeightG = 8;
-template <class T>
+template <int KIND>
 __global__ void __launch_bounds__(kLayerThreads) layer_weight_tiled_kernel(const LayerShape sh,
                                                                            const float *__restrict__ P,
                                                                            const float *__restrict__ Q,
-                                                                           T *__restrict__ W) {
+                                                                           const WeightOut W, int *flag, int epoch) {
   extern __shared__ float sm[];
   const int N0 = sh.n[0], N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
   const int R1 = sh.r1, B = N1 * M1, NP = N0 * N1;
@@ -142,7 +161,10 @@ __global__ void __launch_bounds__(kLayerThreads) layer_weight_tiled_kernel(const
     }
 #pragma unroll
     for (int g = 0; g < kWeightG; ++g)
-      if (g < G) W[(o0 + g) * Nin + i] = from_f32<T>(acc[g]);
+      if (g < G) {
+        put_weight<KIND>(W, (o0 + g) * Nin + i, acc[g]);
+        if (KIND == W_PLANES && no_planes(acc[g])) *flag = epoch;
+      }
   }
 }
 
@@ -515,26 +537,29 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
-cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
-                                cudaStream_t s) {
+template <int KIND>
+cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, const WeightOut &W, int *flag, int epoch,
+                          cudaStream_t s) {
   const long long total = static_cast<long long>(sh.n[0]) * sh.n[1] * sh.n[2] * sh.m[0] * sh.m[1] * sh.m[2];
   const size_t smem = layer_weight_smem(sh);
   if (smem <= kLayerSmemMax) {
     const unsigned grid =
         static_cast<unsigned>(sh.m[0]) * sh.m[1] * ((sh.m[2] + kWeightG - 1) / kWeightG);
-    cudaError_t e;
-    if (W32) {
-      if ((e = allow_smem(layer_weight_tiled_kernel<float>, smem)) != cudaSuccess) return e;
-      layer_weight_tiled_kernel<float><<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W32);
-    } else {
-      if ((e = allow_smem(layer_weight_tiled_kernel<__nv_bfloat16>, smem)) != cudaSuccess) return e;
-      layer_weight_tiled_kernel<__nv_bfloat16><<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W16);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = allow_smem(layer_weight_tiled_kernel<KIND>, smem);
+    if (e != cudaSuccess) return e;
+    layer_weight_tiled_kernel<KIND><<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W, flag, epoch);
+  } else {
+    layer_weight_kernel<KIND><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W, flag, epoch);
   }
-  if (W32) layer_weight_kernel<float><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W32);
-  else layer_weight_kernel<__nv_bfloat16><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W16);
   return cudaGetLastError();
+}
+
+cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
+                                __nv_bfloat16 *W3, long long plane, int *flag, int epoch, cudaStream_t s) {
+  const WeightOut W{W32, W16, W3, plane};
+  if (W3) return W32 && flag ? weight_launch<W_PLANES>(sh, P, Q, W, flag, epoch, s) : cudaErrorInvalidValue;
+  if (W32) return weight_launch<W_FP32>(sh, P, Q, W, flag, epoch, s);
+  return weight_launch<W_BF16>(sh, P, Q, W, flag, epoch, s);
 }
 
 cudaError_t bias_act_launch(float *y, const float *bias, long long batch, long long nout, int act, cudaStream_t s) {

@@ -494,7 +494,7 @@ TileGen make_slabs_gen(long long L, long long R, int cols, int bn) {
   return g;
 }
 
-bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g) {
+bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long batch, long long zstride) {
   *g = TileGen{};
   g->kind = TILES_GRID;
   g->bm = 128;
@@ -502,7 +502,12 @@ bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g) {
   g->rows = rows;
   g->n = cols;
   g->cols = bn;
-  const long long count = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
+  if (batch < 1 || batch > 65535 || rows > (1ll << 40) || cols > (1ll << 40)) return false;
+  g->R = batch;
+  g->L = zstride;
+  const long long tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
+  if (tiles > (1ll << 30)) return false;
+  const long long count = tiles * batch;
   if (rows < 1 || cols < 1 || count > (1ll << 30) || rows > (1ll << 31) - 256 || cols > (1ll << 31) - 256) return false;
   g->count = static_cast<int>(count);
   return true;

@@ -59,6 +59,8 @@ struct KParams {
   int fold;
   int same;    // A and B are the same operand: a tile with a_row == b_row loads one panel
   __nv_bfloat16 *out16;   // OUT_COLMAJOR only: write the tile in BF16 here instead of FP32 to out
+  const float *bias;      // OUT_COLMAJOR, FP32: bias[row] added to the row, or null
+  int relu;
 };
 
 // Issue the TMA loads of one operand tile (ROWS x 64 K) for k-block kb.
@@ -219,6 +221,15 @@ HT_DEV void tc_gemm_tile(const CUtensorMap *tmA, const CUtensorMap *tmB, const K
             if (c0 + j < tile.valid_cols) dst[p.ld_out * j] = __float2bfloat16_rn(v[j]);
         } else {
           float *dst = p.out + off;
+          if (p.bias) {
+            const float b = __ldg(p.bias + tile.out_row + row);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += b;
+          }
+          if (p.relu) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+          }
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (c0 + j < tile.valid_cols) dst[p.ld_out * j] = v[j];
@@ -357,6 +368,8 @@ cudaError_t launch_bn(const GemmArgs &g, cudaStream_t s) {
   p.err = g.err;
   p.fold = (g.fold && g.out_mode == OUT_COLMAJOR) ? 1 : 0;
   p.out16 = g.out_mode == OUT_COLMAJOR ? g.out16 : nullptr;
+  p.bias = g.out_mode == OUT_COLMAJOR ? g.bias : nullptr;
+  p.relu = g.out_mode == OUT_COLMAJOR ? g.relu : 0;
   p.same = (g.a.ptr == g.b.ptr && g.a.kind == g.b.kind && g.a.d0 == g.b.d0 && g.a.d1 == g.b.d1 && g.a.d2 == g.b.d2) ? 1 : 0;
   cudaError_t e = set_smem<BN, MT>();
   if (e != cudaSuccess) return e;

@@ -25,10 +25,15 @@ HT_DEV Tile gen_tile(const TileGen &g, int idx) {
     t.valid_cols = min(g.cols, g.bn);
   } else if (g.kind == TILES_GRID) {
     const long long nrb = (g.rows + g.bm - 1) / g.bm;
+    if (g.R > 1) {
+      const long long per = nrb * ((g.n + g.bn - 1) / g.bn);
+      t.a_z = static_cast<int>(idx / per);
+      idx -= static_cast<int>(t.a_z * per);
+    }
     const long long cb = idx / nrb, rb = idx - cb * nrb;
     t.a_row = static_cast<int>(g.bm * rb);
     t.b_row = static_cast<int>(g.bn * cb);
-    t.out_row = g.bm * rb;
+    t.out_row = g.bm * rb + g.L * t.a_z;
     t.out_col = static_cast<int>(g.bn * cb);
     t.valid_rows = static_cast<int>(min(static_cast<long long>(g.bm), g.rows - g.bm * rb));
     t.valid_cols = static_cast<int>(min(static_cast<long long>(g.bn), g.n - g.bn * cb));

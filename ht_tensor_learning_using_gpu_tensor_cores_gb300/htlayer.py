@@ -14,7 +14,7 @@ Mirrors the reference's HT layer (``HT_tensor_layer/FC_MNIST/mnist_ht.py``):
 
 The forward and backward run in ``libhtgb.so`` (``ht_layer_forward`` /
 ``ht_layer_backward``): the weight is formed from the factors on the GPU and
-the batch goes through one GEMM (FP32 SIMT, or tcgen05 on BF16 operands with
+the batch goes through one GEMM (FP32-accurate, or on BF16 operands with
 ``precision="bf16"``).  There is no PyTorch fallback.
 """
 from __future__ import annotations

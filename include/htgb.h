@@ -47,7 +47,8 @@ typedef enum {
 } ht_status_t;
 
 typedef enum {
-    HT_PREC_FP32 = 0,  /* plain path: every product in FP32 on CUDA cores          */
+    HT_PREC_FP32 = 0,  /* plain path: every product to FP32 accuracy (CUDA cores, or
+                           three BF16 planes per operand on tcgen05)               */
     HT_PREC_BF16 = 1   /* mixed path: BF16 tcgen05 GEMMs, FP32 accumulation in TMEM */
 } ht_precision_t;
 
@@ -108,7 +109,7 @@ typedef struct {
                                 and stage 2 is empty.                             */
     double eig_residual[HT_MAX_NODES]; /* max_j ||G u_j - theta_j u_j|| / theta_1   */
     int gpu_launches;        /* kernels launched by this call                     */
-    int path_flags;          /* bit 0: tcgen05 path used, bit 1: SIMT path used   */
+    int path_flags;          /* bit 0: BF16 products (tcgen05), bit 1: FP32 ones  */
 } ht_report_t;
 
 /* ------------------------------------------------------------------ setup */
@@ -325,7 +326,7 @@ ht_status_t ht_sketch_adam(float *S, const float *grad, float *m, float *v, long
  * Ranks <= 64.  All pointers are device memory.  The calls are asynchronous on
  * `stream` and use a per-device workspace of their own: calls that may overlap
  * on the GPU (different streams) must be ordered by the caller.
- * precision: HT_PREC_FP32 (FP32 SIMT products) or HT_PREC_BF16 (tcgen05
+ * precision: HT_PREC_FP32 (FP32-accurate products) or HT_PREC_BF16 (tcgen05
  * products on BF16 operands, FP32 accumulation; needs n and m products that are
  * multiples of 8). */
 typedef struct {
