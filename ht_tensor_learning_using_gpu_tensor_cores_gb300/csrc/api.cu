@@ -376,7 +376,8 @@ ht_status_t run_gemm(Ctx &c, const GemmReq &q) {
   if (q.tiles_kind == TILES_ROWS) gen = make_rows_gen(q.t_rows, q.t_cols, bn);
   else if (q.tiles_kind == TILES_SLABS) gen = make_slabs_gen(q.t_L, q.t_R, q.t_cols, bn);
   else if (q.tiles_kind == TILES_GRID) {
-    if (!make_grid_gen(q.t_rows, q.t_n, bn, &gen)) return fail(HT_ERR_UNSUPPORTED, "product too large for one grid");
+    if (!make_grid_gen(q.t_rows, q.t_n, bn, &gen, 1, 0, 128 * mt))
+      return fail(HT_ERR_UNSUPPORTED, "product too large for one grid");
   } else if (!make_gram_gen(q.t_n, bn, &gen, 128 * mt)) return fail(HT_ERR_UNSUPPORTED, "Gram larger than 32768");
   const int nt = gen.count;
   int splits = 1;
@@ -3864,6 +3865,16 @@ ht_status_t layer_gemm(Ctx &c, const Operand &a32, const Operand &b32, const Ope
   q.a16 = a16;
   q.b16 = b16;
   q.bn_tc = cols >= 256 ? 256 : (cols > 64 ? 128 : 64);
+  if (rows >= 256 && cols >= 256) {
+    // 256 x 256 tiles (two accumulators share every B stage) keep the tensor
+    // pipe full where 128 x 256 ones leave it half idle (4096 x 4096 x 6400: 107
+    // against 204 us), so they are taken unless their last wave costs more
+    const long long t1 = ((rows + 127) / 128) * ((cols + 255) / 256), t2 = ((rows + 255) / 256) * ((cols + 255) / 256);
+    auto waves = [](long long t) { return t < sm_count() ? 1.0 : double((t + sm_count() - 1) / sm_count()); };
+    // (too few tiles for the SMs: only where K is long enough to split)
+    const bool few = t1 < sm_count();
+    if (few ? t2 * (a16.ptr ? tc_num_kblocks(a16) / 16 : 0) >= sm_count() : 2.1 * waves(t2) <= 1.9 * waves(t1)) q.mt_tc = 2;
+  }
   q.bn_simt = cols > 64 ? 128 : 64;
   q.tiles_kind = TILES_GRID;
   q.t_rows = rows;
@@ -3999,7 +4010,7 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
       HT_TRY(reserve_planes(c, nout, batch, &dy3));
     }
     if (!c.dry()) {
-      HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, T1, c.st));
+      HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, T1, c.st, dbias ? dy : nullptr, batch, part));
       ++c.launches;
       if (dx) {
         HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.epoch, c.st));
@@ -4029,13 +4040,8 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
     HT_TRY(layer_gemm(c, op_of(OP_MN3, x, nin, batch), op_of(OP_MN3, dy, nout, batch),
                       op_of(OP_MN3, x16, nin, batch), op_of(OP_MN3, dy16, nout, batch), x3, dy3, nin, nout, dW));
     if (!c.dry()) {
-      if (dbias) {
-        HT_CUDA(layer_colsum_launch(dy, batch, nout, part, dbias, c.st));
-        c.launches += 2;
-      }
-      HT_CUDA(layer_factor_grads_launch(sh, dW, u1, u2, u3, b2, b1, P, Q, T1, dP, dQ, dT1, dQpart, du1, du2, du3,
-                                        db2, db1, c.st));
-      c.launches += 4;
+      HT_CUDA(layer_factor_grads_launch(sh, dW, batch, u1, u2, u3, b2, b1, P, Q, T1, dP, dQ, dT1, dQpart, part, du1,
+                                        du2, du3, db2, db1, dbias, c.st, &c.launches));
     }
     return HT_OK;
   });

@@ -178,7 +178,8 @@ cudaError_t reduce_partials_launch(const float *partial, const TileGen &gen, int
 TileGen make_rows_gen(long long rows, int cols, int bn);
 TileGen make_slabs_gen(long long L, long long R, int cols, int bn);
 // rows x cols output in 128 x bn tiles (TILES_GRID); false when the tile count overflows
-bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long batch = 1, long long zstride = 0);
+bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long batch = 1, long long zstride = 0,
+                   int bm = 128);
 bool make_gram_gen(long long n, int bn, TileGen *g, int bm = 128);
 
 // Multiprocessor count of the current device (cached per device).
@@ -445,23 +446,26 @@ struct LayerShape {
 // P[a, b, r1] (A x B x r1), Q[c, r1] (C x r1) and, when T1 is non-null,
 // T1[a, r4, r1] = sum_r3 u1[a, r3] b2[r3, r4, r1]
 cudaError_t layer_pq_launch(const LayerShape &sh, const float *u1, const float *u2, const float *u3, const float *b2,
-                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s);
+                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s, const float *dy = nullptr,
+                            long long batch = 0, float *cpart = nullptr);
 // W (Nout x Nin, row-major) from P and Q, into W32 (FP32) or, when W32 is null, W16 (BF16)
 cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
                                 __nv_bfloat16 *W3, long long plane, int *flag, int epoch, cudaStream_t s);
 // y[z, o] = act(y[z, o] + bias[o]) (bias may be null; act 0 identity, 1 ReLU)
 cudaError_t bias_act_launch(float *y, const float *bias, long long batch, long long nout, int act, cudaStream_t s);
-// out[o] = sum_z dy[z, o]; part holds layer_colsum_chunks(batch) * nout floats
+// Ranges of the batch whose partial column sums of dy layer_factor_grads_launch
+// keeps in cpart (layer_colsum_chunks(batch) * nout floats).
 int layer_colsum_chunks(long long batch);
-cudaError_t layer_colsum_launch(const float *dy, long long batch, long long nout, float *part, float *out,
-                                cudaStream_t s);
 // Floats of the dQ partial buffer layer_factor_grads_launch wants (0: the shape
 // takes the unfused path, which needs none).
 size_t layer_dq_part_count(const LayerShape &sh);
-// du1, du2, du3, db2, db1 from dW (Nout x Nin, row-major), via dP, dQ, dT1 (scratch of P, Q, T1's sizes)
-cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, const float *u1, const float *u2,
-                                      const float *u3, const float *b2, const float *b1, const float *P,
-                                      const float *Q, const float *T1, float *dP, float *dQ, float *dT1, float *dQpart,
-                                      float *du1, float *du2, float *du3, float *db2, float *db1, cudaStream_t s);
+// du1, du2, du3, db2, db1 from dW (Nout x Nin, row-major), via dP, dQ, dT1 (scratch of P, Q, T1's sizes), and
+// dbias (or null) from the partial column sums in cpart, which a layer_pq_launch
+// with dy forms.  *launches is raised by the kernels launched.
+cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, long long batch, const float *u1, const float *u2, const float *u3, const float *b2,
+                                      const float *b1, const float *P, const float *Q, const float *T1, float *dP,
+                                      float *dQ, float *dT1, float *dQpart, float *cpart, float *du1, float *du2,
+                                      float *du3, float *db2, float *db1, float *dbias, cudaStream_t s,
+                                      int *launches);
 
 }  // namespace htgb

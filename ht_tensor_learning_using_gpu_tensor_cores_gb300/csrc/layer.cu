@@ -32,6 +32,27 @@ int grid_for_layer(long long n) {
   return static_cast<int>(g < 1 ? 1 : g);
 }
 
+// dbias[o] = sum_z dy[z, o]: one thread per o, the batch split into `chunks`
+// ranges whose partial sums layer_reduce_kernel adds in a fixed order.
+HT_DEV void layer_colsum_body(const float *__restrict__ dy, long long batch, long long nout, int chunks,
+                              float *__restrict__ part, int blk) {
+  const int gx = static_cast<int>((nout + kLayerThreads - 1) / kLayerThreads), chunk = blk / gx;
+  const long long o = (blk - chunk * gx) * static_cast<long long>(kLayerThreads) + threadIdx.x;
+  if (o >= nout) return;
+  const long long per = (batch + chunks - 1) / chunks;
+  const long long z0 = per * chunk, z1 = min(batch, z0 + per);
+  float s = 0.f;
+  for (long long z = z0; z < z1; ++z) s += dy[z * nout + o];
+  part[static_cast<long long>(chunk) * nout + o] = s;
+}
+struct ColsumArgs {
+  const float *dy;   // null: none
+  long long batch, nout;
+  int chunks;
+  float *part;
+};
+
+// Blocks past P's and Q's: the column sums of a backward's dy, which ride along.
 // Blocks [0, A): T1[a] = u1[a, :] b2 (r4 x r1, in shared memory, also written to
 // T1g when non-null), then P[a, b, r1] for every b.  Blocks [A, A + qb): Q.
 __global__ void __launch_bounds__(kLayerThreads) layer_pq_kernel(const LayerShape sh, const float *__restrict__ u1,
@@ -39,7 +60,12 @@ __global__ void __launch_bounds__(kLayerThreads) layer_pq_kernel(const LayerShap
                                                                  const float *__restrict__ u3,
                                                                  const float *__restrict__ b2,
                                                                  const float *__restrict__ b1, float *__restrict__ P,
-                                                                 float *__restrict__ Q, float *__restrict__ T1g) {
+                                                                 float *__restrict__ Q, float *__restrict__ T1g,
+                                                                 int npq, const ColsumArgs cs) {
+  if (static_cast<int>(blockIdx.x) >= npq) {
+    layer_colsum_body(cs.dy, cs.batch, cs.nout, cs.chunks, cs.part, blockIdx.x - npq);
+    return;
+  }
   __shared__ float T1[kLayerMaxRank * kLayerMaxRank];
   const int A = sh.n[0] * sh.m[0], B = sh.n[1] * sh.m[1], C = sh.n[2] * sh.m[2];
   const int R1 = sh.r1, R2 = sh.r2, R3 = sh.r3, R4 = sh.r4;
@@ -117,55 +143,76 @@ __global__ void __launch_bounds__(kLayerThreads) layer_weight_kernel(const Layer
   }
 }
 
-// The same W, a block per (m0, m1, group of kWeightG m2 rows): the P slice
-// Ps[(n0, n1)][r] = P[n0 M0 + m0, n1 M1 + m1, r] and Qt[r][g][n2] =
-// Q[n2 M2 + m2_0 + g, r] sit in shared memory, each thread keeps kWeightG
-// accumulators for one input index i and writes kWeightG rows of W, consecutive
-// threads on consecutive i (coalesced rows).
-constexpr int kWeightG = 8;
-template <int KIND>
-__global__ void __launch_bounds__(kLayerThreads) layer_weight_tiled_kernel(const LayerShape sh,
+// The same W, a block per (m0, m1, group of G m2 rows): a thread keeps its n2 and
+// the G x RB entries Q[n2 M2 + m2, :] in registers and walks the pairs, whose
+// rows Ps[(n0, n1)][:] of P sit in shared memory: RB / 4 (broadcast) vector loads
+// for G x RB multiply-adds, so the FMA pipe is the bound; with Q in shared memory
+// its loads were (4096 x 6400 in BF16: 80 -> 63 us).  Consecutive threads write
+// consecutive entries of a row.  G x RB = 64: ranks up to 64.
+template <int KIND, int RB>
+__global__ void __launch_bounds__(kLayerThreads, RB < 64 ? 3 : 1) layer_weight_tiled_kernel(const LayerShape sh,
                                                                            const float *__restrict__ P,
                                                                            const float *__restrict__ Q,
                                                                            const WeightOut W, int *flag, int epoch) {
-  extern __shared__ float sm[];
+  constexpr int G = 64 / RB;
+  extern __shared__ __align__(16) float Ps[];   // NP x RB, zero past R1; behind it Qs: N2 rows of 65
   const int N0 = sh.n[0], N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
   const int R1 = sh.r1, B = N1 * M1, NP = N0 * N1;
   const long long Nin = static_cast<long long>(NP) * N2;
-  const int groups = (M2 + kWeightG - 1) / kWeightG;
+  const int groups = (M2 + G - 1) / G;
   const int gi = blockIdx.x % groups, mm = blockIdx.x / groups, m1 = mm % M1, m0 = mm / M1;
-  const int m2_0 = gi * kWeightG, G = min(kWeightG, M2 - m2_0);
-  float *Ps = sm;                                    // NP x R1
-  float *Qt = sm + static_cast<size_t>(NP) * R1;     // R1 x kWeightG x N2
-  for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
-    const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
-    Ps[e] = P[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r];
+  const int m2_0 = gi * G, ng = min(G, M2 - m2_0);
+  for (int e = threadIdx.x; e < NP * RB; e += kLayerThreads) {
+    const int pr = e / RB, r = e % RB, n0 = pr / N1, n1 = pr - n0 * N1;
+    Ps[e] = r < R1 ? P[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r] : 0.f;
   }
-  for (int e = threadIdx.x; e < R1 * kWeightG * N2; e += kLayerThreads) {
-    const int n2 = e % N2, g = (e / N2) % kWeightG, r = e / (N2 * kWeightG);
-    Qt[e] = g < G ? Q[static_cast<long long>(n2 * M2 + m2_0 + g) * R1 + r] : 0.f;
+  // Q's rows are G R1 contiguous entries a n2: read along them, then a row per thread
+  float *Qs = Ps + NP * RB;
+  for (int e = threadIdx.x; e < N2 * 64; e += kLayerThreads) {
+    const int n2 = e / 64, g = (e % 64) / RB, r = e % RB;
+    Qs[n2 * 65 + (e % 64)] = g < ng && r < R1 ? Q[static_cast<long long>(n2 * M2 + m2_0 + g) * R1 + r] : 0.f;
   }
   __syncthreads();
-  const long long o0 = (static_cast<long long>(m0) * M1 + m1) * M2 + m2_0;
-  for (long long i = threadIdx.x; i < Nin; i += kLayerThreads) {
-    const int pr = static_cast<int>(i / N2), n2 = static_cast<int>(i - static_cast<long long>(pr) * N2);
-    float acc[kWeightG];
+  const long long o0 = ((static_cast<long long>(m0) * M1 + m1) * M2 + m2_0) * Nin;
+  bool bad = false;
+  // columns of n2 in turn where a mode is wider than the block
+  const int nw = min(N2, kLayerThreads), per = kLayerThreads / nw;   // pairs per sweep of the block
+  const int pl = threadIdx.x / nw, nl = threadIdx.x - pl * nw;
+  for (int n2 = nl; n2 < N2 && pl < per; n2 += nw) {
+    constexpr int GP = (G + 1) / 2;   // rows in pairs (RB = 64: one row, its pair's second half idle)
+    float2 q[RB][GP];
 #pragma unroll
-    for (int g = 0; g < kWeightG; ++g) acc[g] = 0.f;
-    const float *ps = Ps + static_cast<size_t>(pr) * R1;
-    for (int r = 0; r < R1; ++r) {
-      const float pv = ps[r];
-      const float *q = Qt + static_cast<size_t>(r) * kWeightG * N2 + n2;
+    for (int r = 0; r < RB; ++r)
 #pragma unroll
-      for (int g = 0; g < kWeightG; ++g) acc[g] = fmaf(pv, q[g * N2], acc[g]);
-    }
+      for (int g = 0; g < GP; ++g)
+        q[r][g] = make_float2(Qs[n2 * 65 + 2 * g * RB + r], 2 * g + 1 < G ? Qs[n2 * 65 + (2 * g + 1) * RB + r] : 0.f);
+    for (int p = pl; p < NP; p += per) {
+      float2 acc[GP];
 #pragma unroll
-    for (int g = 0; g < kWeightG; ++g)
-      if (g < G) {
-        put_weight<KIND>(W, (o0 + g) * Nin + i, acc[g]);
-        if (KIND == W_PLANES && no_planes(acc[g])) *flag = epoch;
+      for (int g = 0; g < GP; ++g) acc[g] = make_float2(0.f, 0.f);
+      const float4 *ps = reinterpret_cast<const float4 *>(Ps + p * RB);
+#pragma unroll
+      for (int r = 0; r < RB; r += 4) {
+        const float4 v = ps[r / 4];
+#pragma unroll
+        for (int g = 0; g < GP; ++g) {
+          fma2(acc[g], make_float2(v.x, v.x), q[r][g]);
+          fma2(acc[g], make_float2(v.y, v.y), q[r + 1][g]);
+          fma2(acc[g], make_float2(v.z, v.z), q[r + 2][g]);
+          fma2(acc[g], make_float2(v.w, v.w), q[r + 3][g]);
+        }
       }
+      const long long i = o0 + static_cast<long long>(p) * N2 + n2;
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (g < ng) {
+          const float v = g & 1 ? acc[g / 2].y : acc[g / 2].x;
+          put_weight<KIND>(W, i + g * Nin, v);
+          bad |= KIND == W_PLANES && no_planes(v);
+        }
+    }
   }
+  if (KIND == W_PLANES && bad) *flag = epoch;
 }
 
 // y[z, o] = act(y[z, o] + bias[o]), act 0 = identity, 1 = ReLU
@@ -178,28 +225,6 @@ __global__ void bias_act_kernel(float *__restrict__ y, const float *__restrict__
     if (act == 1) v = fmaxf(v, 0.f);
     y[e] = v;
   }
-}
-
-// dbias[o] = sum_z dy[z, o]: one thread per o, the batch split over blockIdx.y
-// partials summed in a fixed order by layer_colsum_finish_kernel.
-__global__ void layer_colsum_kernel(const float *__restrict__ dy, long long batch, long long nout, int chunks,
-                                    float *__restrict__ part) {
-  const long long o = blockIdx.x * static_cast<long long>(kLayerThreads) + threadIdx.x;
-  if (o >= nout) return;
-  const long long per = (batch + chunks - 1) / chunks;
-  const long long z0 = per * blockIdx.y, z1 = min(batch, z0 + per);
-  float s = 0.f;
-  for (long long z = z0; z < z1; ++z) s += dy[z * nout + o];
-  part[static_cast<long long>(blockIdx.y) * nout + o] = s;
-}
-
-__global__ void layer_colsum_finish_kernel(const float *__restrict__ part, long long nout, int chunks,
-                                           float *__restrict__ out) {
-  const long long o = blockIdx.x * static_cast<long long>(kLayerThreads) + threadIdx.x;
-  if (o >= nout) return;
-  float s = 0.f;
-  for (int c = 0; c < chunks; ++c) s += part[static_cast<long long>(c) * nout + o];
-  out[o] = s;
 }
 
 // dP[a, b, r1] = sum_{n2, m2} dW[o, i] Q[c, r1] and, in the same pass over dW,
@@ -272,79 +297,165 @@ __global__ void __launch_bounds__(kLayerThreads) layer_dq_kernel(const LayerShap
 // reads its rows o = (m0 M1 + m1) M2 + m2 of dW (coalesced, staged in
 // shared memory with an odd pair stride), and with Q (C x R1) and the P slice
 // Ps[(n0, n1)][r] resident accumulates
-//   dPs[(n0, n1)][r] += sum_n2 dW[o, (n0, n1, n2)] Q[n2 M2 + m2, r]
+//   dPs[r][(n0, n1)] += sum_n2 dW[o, (n0, n1, n2)] Q[n2 M2 + m2, r]
 //   dQpart[blk][n2 M2 + m2][r] = sum_(n0, n1) dW[o, (n0, n1, n2)] Ps[(n0, n1)][r].
-// Every accumulator has one owning thread, so the sums are deterministic.
+// Bound by shared-memory loads, so both products keep a row of outputs in
+// registers: dP a thread per pair and RT ranks (one load of the row and RT / 4
+// broadcast vectors of Q for RT multiply-adds), dQ a lane per n2 and 16 ranks
+// with the pairs spread over the warps (and, for N2 <= 16, over groups of
+// lanes), whose partial sums are added in warp order.  With one output per
+// thread and two loads per multiply-add the pass over a 6400 x 4096 dW took 454
+// us; now 145.  Every sum has a fixed order.
+constexpr int kDqRanks = 16;
+constexpr int kDqRed = 17;   // floats per lane of the partial sums (odd: no bank conflicts)
+template <int RT>
 __global__ void __launch_bounds__(kLayerThreads) layer_dpq_kernel(const LayerShape sh, const float *__restrict__ dW,
                                                                   const float *__restrict__ P,
                                                                   const float *__restrict__ Q,
                                                                   float *__restrict__ dP,
                                                                   float *__restrict__ dQpart) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int N0 = sh.n[0], N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
-  const int R1 = sh.r1, B = N1 * M1, NP = N0 * N1, C = N2 * M2;
+  const int R1 = sh.r1, RP = (R1 + 3) & ~3, B = N1 * M1, NP = N0 * N1, C = N2 * M2;
   const int rs = N2 | 1;                             // odd stride between pairs: conflict-free column reads
   const long long Nin = static_cast<long long>(NP) * N2;
-  const int chunks = gridDim.x / (M0 * M1);          // m2 ranges per (m0, m1): dP partials per range
+  const int chunks = gridDim.x / (M0 * M1);             // m2 ranges per (m0, m1): dP partials per range
   const int blk = blockIdx.x / chunks, ch = blockIdx.x - blk * chunks, m1 = blk % M1, m0 = blk / M1;
   const int mg = (M2 + chunks - 1) / chunks, m2_lo = ch * mg, m2_hi = min(M2, m2_lo + mg);
-  float *row = sm;                                   // NP x rs
-  float *Qs = row + static_cast<size_t>(NP) * rs;    // C x R1
-  float *Ps = Qs + static_cast<size_t>(C) * R1;      // NP x R1
-  float *dPs = Ps + static_cast<size_t>(NP) * R1;    // NP x R1
-  for (int e = threadIdx.x; e < C * R1; e += kLayerThreads) Qs[e] = Q[e];
-  for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
-    const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
-    Ps[e] = P[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r];
-    dPs[e] = 0.f;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  float *Qs = sm;                                              // C x RP
+  float *Ps = Qs + static_cast<size_t>(C) * RP;                // NP x RP, then 64 spare floats
+  float *dPs = Ps + static_cast<size_t>(NP) * RP + 64;         // R1 x NP
+  float *red = dPs + static_cast<size_t>(R1) * NP;             // 256 x kDqRed
+  float *row = red + kLayerThreads * kDqRed;                   // NP x rs
+  for (int e = t; e < C * RP; e += kLayerThreads) {
+    const int c = e / RP, r = e - c * RP;
+    Qs[e] = r < R1 ? Q[static_cast<long long>(c) * R1 + r] : 0.f;
   }
+  for (int e = t; e < NP * RP; e += kLayerThreads) {
+    const int pr = e / RP, r = e - pr * RP, n0 = pr / N1, n1 = pr - n0 * N1;
+    Ps[e] = r < R1 ? P[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r] : 0.f;
+  }
+  for (int e = t; e < 64; e += kLayerThreads) Ps[NP * RP + e] = 0.f;
+  for (int e = t; e < NP * R1; e += kLayerThreads) dPs[e] = 0.f;
+  const int dp = kLayerThreads / N2, dn = kLayerThreads - dp * N2;   // steps of (pair, n2) between a thread's entries
+  const int nl = min(N2, 32), psub = 32 / nl, ps = lane / nl, ln = lane - ps * nl;
   for (int m2 = m2_lo; m2 < m2_hi; ++m2) {
     __syncthreads();   // previous row fully consumed (and Qs / Ps written on the first pass)
     const float *src = dW + ((static_cast<long long>(m0) * M1 + m1) * M2 + m2) * Nin;
-    for (long long i = threadIdx.x; i < Nin; i += kLayerThreads) {
-      const int pr = static_cast<int>(i / N2), n2 = static_cast<int>(i - static_cast<long long>(pr) * N2);
-      row[pr * rs + n2] = src[i];
+    int pr = t / N2, n2 = t - pr * N2;
+    for (long long i = t; i < Nin; i += kLayerThreads) {
+      // (asynchronous: every entry of the row is in flight at once)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(row + pr * rs + n2)), "l"(src + i) : "memory");
+      pr += dp;
+      n2 += dn;
+      if (n2 >= N2) {
+        n2 -= N2;
+        ++pr;
+      }
     }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
-      const int pr = e / R1, r = e - pr * R1;
-      const float *rw = row + pr * rs;
-      float s = dPs[e];
-      for (int n2 = 0; n2 < N2; ++n2) s = fmaf(rw[n2], Qs[(n2 * M2 + m2) * R1 + r], s);
-      dPs[e] = s;
-    }
-    for (int e = threadIdx.x; e < N2 * R1; e += kLayerThreads) {
-      const int r = e / N2, n2 = e - r * N2;
-      float s[4] = {0.f, 0.f, 0.f, 0.f};   // four independent chains, combined in a fixed order
-      int pr = 0;
-      for (; pr + 4 <= NP; pr += 4)
+    for (int e = t; e < NP * ((R1 + RT - 1) / RT); e += kLayerThreads) {
+      const int g = e / NP, q = e - g * NP, r0 = g * RT;
+      const float *rw = row + q * rs, *qv = Qs + static_cast<size_t>(m2) * RP + r0;
+      float2 acc[RT / 2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[j] = fmaf(row[(pr + j) * rs + n2], Ps[(pr + j) * R1 + r], s[j]);
-      for (; pr < NP; ++pr) s[0] = fmaf(row[pr * rs + n2], Ps[pr * R1 + r], s[0]);
-      dQpart[(static_cast<long long>(blk) * C + (n2 * M2 + m2)) * R1 + r] = (s[0] + s[1]) + (s[2] + s[3]);
+      for (int r = 0; r < RT / 2; ++r) acc[r] = make_float2(0.f, 0.f);
+      for (int c = 0; c < N2; ++c, qv += static_cast<size_t>(M2) * RP) {
+        const float x = rw[c];
+#pragma unroll
+        for (int r = 0; r < RT; r += 4) {   // (vectors past RP read the next row's: their sums are dropped)
+          const float4 v = *reinterpret_cast<const float4 *>(qv + r);
+          fma2(acc[r / 2], make_float2(x, x), make_float2(v.x, v.y));
+          fma2(acc[r / 2 + 1], make_float2(x, x), make_float2(v.z, v.w));
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        if (r0 + r < R1) dPs[(r0 + r) * NP + q] += r & 1 ? acc[r / 2].y : acc[r / 2].x;
     }
+    for (int nc = 0; nc < N2; nc += 32)
+      for (int r0 = 0; r0 < R1; r0 += kDqRanks) {
+        float2 acc[kDqRanks / 2];
+#pragma unroll
+        for (int r = 0; r < kDqRanks / 2; ++r) acc[r] = make_float2(0.f, 0.f);
+        if (ps < psub && nc + ln < N2) {
+          for (int q = warp * psub + ps; q < NP; q += 8 * psub) {
+            const float x = row[q * rs + nc + ln];
+            const float *pv = Ps + static_cast<size_t>(q) * RP + r0;
+#pragma unroll
+            for (int r = 0; r < kDqRanks; r += 4) {
+              const float4 v = *reinterpret_cast<const float4 *>(pv + r);
+              fma2(acc[r / 2], make_float2(x, x), make_float2(v.x, v.y));
+              fma2(acc[r / 2 + 1], make_float2(x, x), make_float2(v.z, v.w));
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < kDqRanks; ++r) red[t * kDqRed + r] = r & 1 ? acc[r / 2].y : acc[r / 2].x;
+        __syncthreads();
+        const int nn = min(nl, N2 - nc), nr = min(kDqRanks, R1 - r0);
+        for (int e = t; e < nn * nr; e += kLayerThreads) {
+          const int k = e / nr, r = e - k * nr;
+          float s = 0.f;
+          for (int w = 0; w < 8; ++w)
+            for (int g = 0; g < psub; ++g) s += red[(w * 32 + g * nl + k) * kDqRed + r];
+          dQpart[(static_cast<long long>(blk) * C + ((nc + k) * M2 + m2)) * R1 + r0 + r] = s;
+        }
+        __syncthreads();
+      }
   }
   __syncthreads();
   // chunks > 1: dP points at the partial buffer [chunks][A B R1]
   float *dPo = dP + static_cast<long long>(ch) * (static_cast<long long>(sh.n[0]) * M0 * B * R1);
-  for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
+  for (int e = t; e < NP * R1; e += kLayerThreads) {
     const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
-    dPo[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r] = dPs[e];
+    dPo[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r] = dPs[r * NP + pr];
   }
 }
 
-// dQ[c, r] = sum over the (m0, m1) blocks of dQpart, in block order.
-__global__ void layer_dq_reduce_kernel(const float *__restrict__ dQpart, int blocks, long long count,
-                                       float *__restrict__ dQ) {
-  const long long e = blockIdx.x * static_cast<long long>(kLayerThreads) + threadIdx.x;
-  if (e >= count) return;
-  float s[4] = {0.f, 0.f, 0.f, 0.f};   // four independent chains, combined in a fixed order
-  int b = 0;
-  for (; b + 4 <= blocks; b += 4)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s[q] += dQpart[static_cast<long long>(b + q) * count + e];
-  for (; b < blocks; ++b) s[0] += dQpart[static_cast<long long>(b) * count + e];
-  dQ[e] = (s[0] + s[1]) + (s[2] + s[3]);
+// Sums of partials in a fixed order, several arrays in one launch: out[e] = sum
+// over k < n of part[k * count + e].  Few partials (dP): a thread per output.
+// Many (dQ, dbias): 32 outputs a block, each warp one contiguous eighth of the
+// partials, the eighths added in order.
+struct SumJob {
+  const float *part;
+  float *out;
+  long long count;
+  int n, blocks;
+};
+struct SumJobs {
+  SumJob j[3];
+};
+__global__ void __launch_bounds__(kLayerThreads) layer_reduce_kernel(const SumJobs jobs) {
+  __shared__ float red[8][32];
+  int blk = blockIdx.x, i = 0;
+  while (i < 2 && blk >= jobs.j[i].blocks) blk -= jobs.j[i++].blocks;
+  const SumJob J = jobs.j[i];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (J.n < 16) {
+    const long long e = blk * static_cast<long long>(kLayerThreads) + t;
+    if (e >= J.count) return;
+    float s = 0.f;
+    for (int k = 0; k < J.n; ++k) s += J.part[k * J.count + e];
+    J.out[e] = s;
+    return;
+  }
+  const long long e = blk * 32ll + lane;
+  const int per = (J.n + 7) / 8, k1 = min(J.n, (warp + 1) * per);
+  float s = 0.f;
+  if (e < J.count)
+    for (int k = warp * per; k < k1; ++k) s += J.part[k * J.count + e];
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && e < J.count) {
+    for (int w = 1; w < 8; ++w) s += red[w][lane];
+    J.out[e] = s;
+  }
+}
+int sum_blocks(int n, long long count) {
+  return static_cast<int>(n < 16 ? (count + kLayerThreads - 1) / kLayerThreads : (count + 31) / 32);
 }
 
 // dT1[a, r4, r1] = sum_b u2[b, r4] dP[a, b, r1]: a block per a, the b range
@@ -352,15 +463,13 @@ __global__ void layer_dq_reduce_kernel(const float *__restrict__ dQpart, int blo
 // each thread owning fixed (r4, r1) outputs.  Blocks [A, A + du3 blocks):
 // du3[c, r2] = sum_r1 dQ[c, r1] b1[r1, r2], a thread per entry.
 constexpr int kDtChunk = 64;
-__global__ void __launch_bounds__(kLayerThreads) layer_dt1_kernel(const LayerShape sh, const float *__restrict__ u2,
-                                                                  const float *__restrict__ b1,
-                                                                  const float *__restrict__ dP,
-                                                                  const float *__restrict__ dQ,
-                                                                  float *__restrict__ dT1, float *__restrict__ du3) {
+HT_DEV void layer_dt1_body(const LayerShape &sh, const float *__restrict__ u2, const float *__restrict__ b1,
+                           const float *__restrict__ dP, const float *__restrict__ dQ, float *__restrict__ dT1,
+                           float *__restrict__ du3, int blk, float *smem) {
   const int A = sh.n[0] * sh.m[0], B = sh.n[1] * sh.m[1], C = sh.n[2] * sh.m[2];
   const int R1 = sh.r1, R2 = sh.r2, R4 = sh.r4, t = threadIdx.x;
-  if (static_cast<int>(blockIdx.x) >= A) {
-    const long long f = (blockIdx.x - A) * static_cast<long long>(kLayerThreads) + t;
+  if (static_cast<int>(blk) >= A) {
+    const long long f = (blk - A) * static_cast<long long>(kLayerThreads) + t;
     if (f >= static_cast<long long>(C) * R2) return;
     const int c = static_cast<int>(f / R2), r2 = static_cast<int>(f - static_cast<long long>(c) * R2);
     float v = 0.f;
@@ -368,10 +477,10 @@ __global__ void __launch_bounds__(kLayerThreads) layer_dt1_kernel(const LayerSha
     du3[f] = v;
     return;
   }
-  __shared__ float sP[kDtChunk * kLayerMaxRank];   // [b][r1]
-  __shared__ float sU[kDtChunk * kLayerMaxRank];   // [b][r4]
+  float *sP = smem;                                  // [b][r1]
+  float *sU = smem + kDtChunk * kLayerMaxRank;       // [b][r4]
   constexpr int kOut = kLayerMaxRank * kLayerMaxRank / kLayerThreads;
-  const int a = blockIdx.x, nout = R4 * R1;
+  const int a = blk, nout = R4 * R1;
   float acc[kOut];
 #pragma unroll
   for (int q = 0; q < kOut; ++q) acc[q] = 0.f;
@@ -440,17 +549,17 @@ __global__ void __launch_bounds__(kLayerThreads) layer_dt1_back_kernel(const Lay
 //   dT1[a, r4, r1] = sum_b dP[a, b, r1] u2[b, r4]   du2[b, r4] = sum_{a, r1} dP[a, b, r1] T1[a, r4, r1]
 //   du1[a, r3] = sum_{r4, r1} dT1[a, r4, r1] b2[r3, r4, r1]
 //   db2[r3, r4, r1] = sum_a u1[a, r3] dT1[a, r4, r1]
-// dT1 and du3 come from layer_dt1_kernel, du1 and db2 from
-// layer_dt1_back_kernel, du2 and db1 from the two kernels below.
+// dT1, du3, du2 and db1 come from layer_grads_kernel, a block range each; du1 and
+// db2, which need all of dT1, from layer_dt1_back_kernel.
 // du2[b, r4] = sum_{a, r1} dP[a, b, r1] T1[a, r4, r1]: a block per b, the
 // (a, r1) pairs split over the threads with R4 accumulators each, then a
 // fixed-order reduction (deterministic).
 template <int RB>   // rank bound: R4 <= RB
-__global__ void __launch_bounds__(kLayerThreads) layer_du2_kernel(const LayerShape sh, const float *__restrict__ dP,
-                                                                  const float *__restrict__ T1, float *__restrict__ du2) {
-  __shared__ float red[kLayerThreads / 32][RB];
+HT_DEV void layer_du2_body(const LayerShape &sh, const float *__restrict__ dP, const float *__restrict__ T1,
+                           float *__restrict__ du2, int blk, float *smem) {
+  float (*red)[RB] = reinterpret_cast<float (*)[RB]>(smem);
   const int A = sh.n[0] * sh.m[0], B = sh.n[1] * sh.m[1];
-  const int R1 = sh.r1, R4 = sh.r4, b = blockIdx.x;
+  const int R1 = sh.r1, R4 = sh.r4, b = blk;
   float acc[RB];
 #pragma unroll
   for (int r = 0; r < RB; ++r) acc[r] = 0.f;
@@ -480,10 +589,10 @@ __global__ void __launch_bounds__(kLayerThreads) layer_du2_kernel(const LayerSha
 // db1[r1, r2] = sum_c dQ[c, r1] u3[c, r2]: a block per r1, c split over the
 // threads with R2 accumulators each, fixed-order reduction.
 template <int RB>   // rank bound: R2 <= RB
-__global__ void __launch_bounds__(kLayerThreads) layer_db1_kernel(const LayerShape sh, const float *__restrict__ dQ,
-                                                                  const float *__restrict__ u3, float *__restrict__ db1) {
-  __shared__ float red[kLayerThreads / 32][RB];
-  const int C = sh.n[2] * sh.m[2], R1 = sh.r1, R2 = sh.r2, r1 = blockIdx.x;
+HT_DEV void layer_db1_body(const LayerShape &sh, const float *__restrict__ dQ, const float *__restrict__ u3,
+                           float *__restrict__ db1, int blk, float *smem) {
+  float (*red)[RB] = reinterpret_cast<float (*)[RB]>(smem);
+  const int C = sh.n[2] * sh.m[2], R1 = sh.r1, R2 = sh.r2, r1 = blk;
   float acc[RB];
 #pragma unroll
   for (int r = 0; r < RB; ++r) acc[r] = 0.f;
@@ -509,27 +618,51 @@ __global__ void __launch_bounds__(kLayerThreads) layer_db1_kernel(const LayerSha
   }
 }
 
+template <int RB>   // rank bound: R2, R4 <= RB
+__global__ void __launch_bounds__(kLayerThreads) layer_grads_kernel(const LayerShape sh, const float *__restrict__ u2,
+                                                                    const float *__restrict__ u3,
+                                                                    const float *__restrict__ b1,
+                                                                    const float *__restrict__ T1,
+                                                                    const float *__restrict__ dP,
+                                                                    const float *__restrict__ dQ,
+                                                                    float *__restrict__ dT1, float *__restrict__ du2,
+                                                                    float *__restrict__ du3, float *__restrict__ db1,
+                                                                    int nb_du2, int nb_dt1) {
+  __shared__ float smem[2 * kDtChunk * kLayerMaxRank];
+  const int blk = blockIdx.x;
+  if (blk < nb_du2) layer_du2_body<RB>(sh, dP, T1, du2, blk, smem);
+  else if (blk < nb_du2 + nb_dt1) layer_dt1_body(sh, u2, b1, dP, dQ, dT1, du3, blk - nb_du2, smem);
+  else layer_db1_body<RB>(sh, dQ, u3, db1, blk - nb_du2 - nb_dt1, smem);
+}
+
 }  // namespace
 
 cudaError_t layer_pq_launch(const LayerShape &sh, const float *u1, const float *u2, const float *u3, const float *b2,
-                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s) {
+                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s, const float *dy,
+                            long long batch, float *cpart) {
   const int A = sh.n[0] * sh.m[0], C = sh.n[2] * sh.m[2];
   const long long qb = (static_cast<long long>(C) * sh.r1 + kLayerThreads - 1) / kLayerThreads;
-  layer_pq_kernel<<<static_cast<unsigned>(A + qb), kLayerThreads, 0, s>>>(sh, u1, u2, u3, b2, b1, P, Q, T1);
+  const ColsumArgs cs{dy, batch, static_cast<long long>(sh.m[0]) * sh.m[1] * sh.m[2], layer_colsum_chunks(batch), cpart};
+  const long long ncol = dy ? (cs.nout + kLayerThreads - 1) / kLayerThreads * cs.chunks : 0;
+  layer_pq_kernel<<<static_cast<unsigned>(A + qb + ncol), kLayerThreads, 0, s>>>(sh, u1, u2, u3, b2, b1, P, Q, T1,
+                                                                                static_cast<int>(A + qb), cs);
   return cudaGetLastError();
 }
 
+// Rank bound of the tiled weight kernel's instantiation.
+int layer_weight_rb(const LayerShape &sh) { return sh.r1 <= 16 ? 16 : (sh.r1 <= 32 ? 32 : 64); }
 size_t layer_weight_smem(const LayerShape &sh) {
-  return sizeof(float) * (static_cast<size_t>(sh.n[0]) * sh.n[1] * sh.r1 +
-                          static_cast<size_t>(sh.r1) * kWeightG * sh.n[2]);
+  return sizeof(float) * (static_cast<size_t>(sh.n[0]) * sh.n[1] * layer_weight_rb(sh) + static_cast<size_t>(sh.n[2]) * 65);
 }
 
 size_t layer_dpq_smem(const LayerShape &sh) {
   const size_t NP = static_cast<size_t>(sh.n[0]) * sh.n[1], C = static_cast<size_t>(sh.n[2]) * sh.m[2];
-  return sizeof(float) * (NP * (sh.n[2] | 1) + C * sh.r1 + 2 * NP * sh.r1);
+  const size_t RP = (sh.r1 + 3) & ~3;
+  return sizeof(float) *
+         (NP * (sh.n[2] | 1) + C * RP + NP * RP + 64 + NP * sh.r1 + static_cast<size_t>(kLayerThreads) * kDqRed);
 }
 
-constexpr size_t kLayerSmemMax = 200 * 1024;
+constexpr size_t kLayerSmemMax = 200 * 1024, kDpqSmemMax = 224 * 1024;
 
 template <class K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
@@ -543,11 +676,17 @@ cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, 
   const long long total = static_cast<long long>(sh.n[0]) * sh.n[1] * sh.n[2] * sh.m[0] * sh.m[1] * sh.m[2];
   const size_t smem = layer_weight_smem(sh);
   if (smem <= kLayerSmemMax) {
-    const unsigned grid =
-        static_cast<unsigned>(sh.m[0]) * sh.m[1] * ((sh.m[2] + kWeightG - 1) / kWeightG);
-    const cudaError_t e = allow_smem(layer_weight_tiled_kernel<KIND>, smem);
+    const int rb = layer_weight_rb(sh), G = 64 / rb;
+    const unsigned grid = static_cast<unsigned>(sh.m[0]) * sh.m[1] * ((sh.m[2] + G - 1) / G);
+    auto launch = [&](auto kernel) -> cudaError_t {
+      const cudaError_t e = allow_smem(kernel, smem);
+      if (e == cudaSuccess) kernel<<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W, flag, epoch);
+      return e;
+    };
+    const cudaError_t e = rb == 16   ? launch(layer_weight_tiled_kernel<KIND, 16>)
+                          : rb == 32 ? launch(layer_weight_tiled_kernel<KIND, 32>)
+                                     : launch(layer_weight_tiled_kernel<KIND, 64>);
     if (e != cudaSuccess) return e;
-    layer_weight_tiled_kernel<KIND><<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W, flag, epoch);
   } else {
     layer_weight_kernel<KIND><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W, flag, epoch);
   }
@@ -574,69 +713,79 @@ int layer_colsum_chunks(long long batch) {
   return static_cast<int>(c);
 }
 
-cudaError_t layer_colsum_launch(const float *dy, long long batch, long long nout, float *part, float *out,
-                                cudaStream_t s) {
-  const int chunks = layer_colsum_chunks(batch);
-  const unsigned gx = static_cast<unsigned>((nout + kLayerThreads - 1) / kLayerThreads);
-  layer_colsum_kernel<<<dim3(gx, chunks), kLayerThreads, 0, s>>>(dy, batch, nout, chunks, part);
-  layer_colsum_finish_kernel<<<gx, kLayerThreads, 0, s>>>(part, nout, chunks, out);
-  return cudaGetLastError();
-}
-
 int layer_dpq_chunks(const LayerShape &sh) {
   const int blocks = sh.m[0] * sh.m[1];
-  int ch = (2 * device_sm_count() + blocks - 1) / blocks;
+  int ch = (3 * device_sm_count() / 2 + blocks - 1) / blocks;   // two blocks an SM, in one wave
   return ch < 1 ? 1 : (ch > sh.m[2] ? sh.m[2] : ch);
 }
 
 size_t layer_dq_part_count(const LayerShape &sh) {
-  if (layer_dpq_smem(sh) > kLayerSmemMax) return 0;
+  if (layer_dpq_smem(sh) > kDpqSmemMax) return 0;
   const size_t dq = static_cast<size_t>(sh.m[0]) * sh.m[1] * sh.n[2] * sh.m[2] * sh.r1;
   const int ch = layer_dpq_chunks(sh);
   const size_t dp = ch > 1 ? static_cast<size_t>(ch) * sh.n[0] * sh.m[0] * sh.n[1] * sh.m[1] * sh.r1 : 0;
   return dq + dp;   // dQ partials, then dP partials
 }
 
-cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, const float *u1, const float *u2,
-                                      const float *u3, const float *b2, const float *b1, const float *P,
-                                      const float *Q, const float *T1, float *dP, float *dQ, float *dT1, float *dQpart,
-                                      float *du1, float *du2, float *du3, float *db2, float *db1, cudaStream_t s) {
-  const int A = sh.n[0] * sh.m[0], B = sh.n[1] * sh.m[1], C = sh.n[2] * sh.m[2];
+cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, long long batch, const float *u1, const float *u2, const float *u3, const float *b2,
+                                      const float *b1, const float *P, const float *Q, const float *T1, float *dP,
+                                      float *dQ, float *dT1, float *dQpart, float *cpart, float *du1, float *du2,
+                                      float *du3, float *db2, float *db1, float *dbias, cudaStream_t s,
+                                      int *launches) {
+  const int A = sh.n[0] * sh.m[0], B = sh.n[1] * sh.m[1], C = sh.n[2] * sh.m[2], NP = sh.n[0] * sh.n[1];
+  const long long nout = static_cast<long long>(sh.m[0]) * sh.m[1] * sh.m[2];
+  const int cchunks = layer_colsum_chunks(batch);
   const size_t smem_dpq = layer_dpq_smem(sh);
-  if (smem_dpq <= kLayerSmemMax && dQpart) {
-    cudaError_t e = allow_smem(layer_dpq_kernel, smem_dpq);
-    if (e != cudaSuccess) return e;
+  SumJobs sums{};
+  cudaError_t e;
+  if (smem_dpq <= kDpqSmemMax && dQpart) {
     const int blocks = sh.m[0] * sh.m[1], ch = layer_dpq_chunks(sh);
-    float *dPpart = dQpart + static_cast<size_t>(blocks) * C * sh.r1;
-    layer_dpq_kernel<<<static_cast<unsigned>(blocks * ch), kLayerThreads, smem_dpq, s>>>(sh, dW, P, Q,
-                                                                                         ch > 1 ? dPpart : dP, dQpart);
-    const long long cnt = static_cast<long long>(C) * sh.r1;
-    layer_dq_reduce_kernel<<<static_cast<unsigned>((cnt + kLayerThreads - 1) / kLayerThreads), kLayerThreads, 0, s>>>(
-        dQpart, blocks, cnt, dQ);
-    if (ch > 1) {
-      const long long pc = static_cast<long long>(A) * B * sh.r1;
-      layer_dq_reduce_kernel<<<static_cast<unsigned>((pc + kLayerThreads - 1) / kLayerThreads), kLayerThreads, 0,
-                               s>>>(dPpart, ch, pc, dP);
-    }
+    float *dPpart = dQpart + static_cast<size_t>(blocks) * C * sh.r1, *dPo = ch > 1 ? dPpart : dP;
+    // ranks per thread: as many as leave every thread a pair
+    auto launch = [&](auto kernel) -> cudaError_t {
+      const cudaError_t r = allow_smem(kernel, smem_dpq);
+      if (r != cudaSuccess) return r;
+      kernel<<<static_cast<unsigned>(blocks * ch), kLayerThreads, smem_dpq, s>>>(sh, dW, P, Q, dPo, dQpart);
+      return cudaGetLastError();
+    };
+    if (NP * ((sh.r1 + 15) / 16) >= kLayerThreads) e = launch(layer_dpq_kernel<16>);
+    else if (NP * ((sh.r1 + 7) / 8) >= kLayerThreads) e = launch(layer_dpq_kernel<8>);
+    else e = launch(layer_dpq_kernel<4>);
+    if (e != cudaSuccess) return e;
+    const long long cnt = static_cast<long long>(C) * sh.r1, pc = static_cast<long long>(A) * B * sh.r1;
+    sums.j[0] = SumJob{dQpart, dQ, cnt, blocks, sum_blocks(blocks, cnt)};
+    if (ch > 1) sums.j[1] = SumJob{dPpart, dP, pc, ch, sum_blocks(ch, pc)};
+    *launches += 1;
   } else {
     const size_t smem = sizeof(float) * static_cast<size_t>(C);
     if (smem > 48 * 1024) return cudaErrorInvalidValue;
     layer_dp_kernel<<<static_cast<unsigned>(A * B), kLayerThreads, smem, s>>>(sh, dW, Q, dP);
     layer_dq_kernel<<<static_cast<unsigned>(C), kLayerThreads, 0, s>>>(sh, dW, P, dQ);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    *launches += 2;
   }
-  const long long du3_blocks = (static_cast<long long>(C) * sh.r2 + kLayerThreads - 1) / kLayerThreads;
-  layer_dt1_kernel<<<static_cast<unsigned>(A + du3_blocks), kLayerThreads, 0, s>>>(sh, u2, b1, dP, dQ, dT1, du3);
-  if (sh.r4 <= 16) layer_du2_kernel<16><<<static_cast<unsigned>(B), kLayerThreads, 0, s>>>(sh, dP, T1, du2);
-  else if (sh.r4 <= 32) layer_du2_kernel<32><<<static_cast<unsigned>(B), kLayerThreads, 0, s>>>(sh, dP, T1, du2);
-  else layer_du2_kernel<kLayerMaxRank><<<static_cast<unsigned>(B), kLayerThreads, 0, s>>>(sh, dP, T1, du2);
-  if (sh.r2 <= 16) layer_db1_kernel<16><<<static_cast<unsigned>(sh.r1), kLayerThreads, 0, s>>>(sh, dQ, u3, db1);
-  else if (sh.r2 <= 32) layer_db1_kernel<32><<<static_cast<unsigned>(sh.r1), kLayerThreads, 0, s>>>(sh, dQ, u3, db1);
-  else layer_db1_kernel<kLayerMaxRank><<<static_cast<unsigned>(sh.r1), kLayerThreads, 0, s>>>(sh, dQ, u3, db1);
+  if (dbias) sums.j[2] = SumJob{cpart, dbias, nout, cchunks, sum_blocks(cchunks, nout)};
+  const int nsum = sums.j[0].blocks + sums.j[1].blocks + sums.j[2].blocks;
+  if (nsum > 0) {
+    layer_reduce_kernel<<<nsum, kLayerThreads, 0, s>>>(sums);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    *launches += 1;
+  }
+  const int du3_blocks = static_cast<int>((static_cast<long long>(C) * sh.r2 + kLayerThreads - 1) / kLayerThreads);
+  const unsigned grid = static_cast<unsigned>(B + A + du3_blocks + sh.r1);
+  const int rb = sh.r4 > sh.r2 ? sh.r4 : sh.r2;
+  auto grads = [&](auto kernel) {
+    kernel<<<grid, kLayerThreads, 0, s>>>(sh, u2, u3, b1, T1, dP, dQ, dT1, du2, du3, db1, B, A + du3_blocks);
+  };
+  if (rb <= 16) grads(layer_grads_kernel<16>);
+  else if (rb <= 32) grads(layer_grads_kernel<32>);
+  else grads(layer_grads_kernel<kLayerMaxRank>);
   const long long du1_blocks = (static_cast<long long>(A) * sh.r3 + kLayerThreads / 32 - 1) / (kLayerThreads / 32);
   const long long db2_blocks =
       (static_cast<long long>(sh.r3) * sh.r4 * sh.r1 + kLayerThreads - 1) / kLayerThreads;
   layer_dt1_back_kernel<<<static_cast<unsigned>(du1_blocks + db2_blocks), kLayerThreads, 0, s>>>(
       sh, u1, b2, dT1, du1, db2, static_cast<int>(du1_blocks));
+  *launches += 2;
   return cudaGetLastError();
 }
 

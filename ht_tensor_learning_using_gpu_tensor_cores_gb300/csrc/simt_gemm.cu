@@ -494,10 +494,10 @@ TileGen make_slabs_gen(long long L, long long R, int cols, int bn) {
   return g;
 }
 
-bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long batch, long long zstride) {
+bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long batch, long long zstride, int bm) {
   *g = TileGen{};
   g->kind = TILES_GRID;
-  g->bm = 128;
+  g->bm = bm;
   g->bn = bn;
   g->rows = rows;
   g->n = cols;
@@ -505,7 +505,7 @@ bool make_grid_gen(long long rows, long long cols, int bn, TileGen *g, long long
   if (batch < 1 || batch > 65535 || rows > (1ll << 40) || cols > (1ll << 40)) return false;
   g->R = batch;
   g->L = zstride;
-  const long long tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
+  const long long tiles = ((rows + bm - 1) / bm) * ((cols + bn - 1) / bn);
   if (tiles > (1ll << 30)) return false;
   const long long count = tiles * batch;
   if (rows < 1 || cols < 1 || count > (1ll << 30) || rows > (1ll << 31) - 256 || cols > (1ll << 31) - 256) return false;
