@@ -2163,7 +2163,8 @@ struct BatchState {
   cudaStream_t lane[kLanes] = {};
   cudaStream_t cap = nullptr;   // capture origin (the caller's stream may be the legacy stream)
   cudaEvent_t fork = nullptr, join[kLanes] = {}, t0 = nullptr, t1 = nullptr;
-  cudaEvent_t tp[5] = {};   // grouped mode: ends of the first five phases (ms_phase)
+  cudaEvent_t tp[2][5] = {};   // grouped mode: ends of the first five phases (ms_phase), of a direct run and of the graph's
+  bool capturing = false;
 
   bool grouped = false;
   double *sums = nullptr;   // device: [count][2] (||X||^2, ||X - Xhat||^2)
@@ -2202,7 +2203,7 @@ struct BatchLayout {
   bool grouped = false;
   size_t lane_bytes = 0;
   std::vector<size_t> off;
-  int nprob = 0, iters = 0, refine = 0;
+  int nprob = 0, nwide = 0, iters = 0, refine = 0;   // leaf problems, those of the 64-wide solver
   int nconv = 0, conv_blocks = 0, ncopy = 0;   // grouped conversion jobs (their blocks), output copies
   int ngram[2] = {0, 0};                       // grouped Grams per class
   int ntail = 0, nerr = 0;                     // grouped transfer tails and error passes
@@ -2238,7 +2239,8 @@ ht_status_t batch_streams(BatchState &b) {
   HT_CUDA(cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
   HT_CUDA(cudaEventCreate(&b.t0));
   HT_CUDA(cudaEventCreate(&b.t1));
-  for (int i = 0; i < 5; ++i) HT_CUDA(cudaEventCreate(&b.tp[i]));
+  for (int w = 0; w < 2; ++w)
+    for (int i = 0; i < 5; ++i) HT_CUDA(cudaEventCreate(&b.tp[w][i]));
 
   return HT_OK;
 }
@@ -2327,6 +2329,14 @@ ht_status_t batch_pass(BatchState &b, const BatchLayout &L, int phase, cudaStrea
   return HT_OK;
 }
 
+// The end of a grouped batch's phase: a plain event record, or inside a capture
+// an external one (an event-record node of the graph).
+ht_status_t batch_phase_end(BatchState &b, int phase, cudaStream_t st) {
+  if (b.capturing) HT_CUDA(cudaEventRecordWithFlags(b.tp[1][phase], st, cudaEventRecordExternal));
+  else HT_CUDA(cudaEventRecord(b.tp[0][phase], st));
+  return HT_OK;
+}
+
 // Enqueue the whole batch on `st`.  Grouped mode: one conversion launch, the
 // grouped Grams, one launch of the grouped leaf solver for every leaf of every
 // tensor (tables uploaded beforehand by batch_plan_grouped), the core pass
@@ -2346,10 +2356,19 @@ ht_status_t batch_enqueue(BatchState &b, const BatchLayout &L, cudaStream_t st, 
   b.launches += (L.ngram[0] > 0) + (L.ngram[1] > 0);
   HT_TRY(batch_pass(b, L, 1, st, count, x, dims, order, trees, cfg, U, B, want_err, eig_ctas));
   // external records: inside a capture they become event-record nodes of the graph
-  HT_CUDA(cudaEventRecordWithFlags(b.tp[0], st, cudaEventRecordExternal));
-  HT_CUDA(eig_grouped_launch(b.table, L.nprob, L.iters, L.refine, st));
-  HT_CUDA(cudaEventRecordWithFlags(b.tp[1], st, cudaEventRecordExternal));
-  b.launches += 1;
+  HT_TRY(batch_phase_end(b, 0, st));
+  // the wide problems (few, long) beside the narrow ones: their CTAs share the SMs
+  if (L.nwide > 0) {
+    HT_CUDA(cudaEventRecord(b.fork, st));
+    HT_CUDA(cudaStreamWaitEvent(b.lane[0], b.fork, 0));
+    HT_CUDA(eig_grouped_launch(b.table, L.nwide, L.nwide, L.iters, L.refine, b.lane[0]));
+    HT_CUDA(cudaEventRecord(b.join[0], b.lane[0]));
+  }
+  HT_CUDA(eig_grouped_launch(static_cast<char *>(b.table) + eig_grouped_entry_bytes() * L.nwide, L.nprob - L.nwide, 0,
+                             L.iters, L.refine, st));
+  if (L.nwide > 0) HT_CUDA(cudaStreamWaitEvent(st, b.join[0], 0));
+  HT_TRY(batch_phase_end(b, 1, st));
+  b.launches += (L.nwide > 0) + (L.nprob > L.nwide);
   if (L.nstep2_blocks > 0) {   // 3rd order: the grouped core pass
     const SParamsBlob *params = static_cast<const SParamsBlob *>(b.core);
     const SimtBlockBlob *tiles =
@@ -2364,10 +2383,10 @@ ht_status_t batch_enqueue(BatchState &b, const BatchLayout &L, cudaStream_t st, 
     b.launches += (L.nnarrow_blocks > 0) + (L.ncore_blocks[0] > 0) + (L.nt1_blocks > 0) + (L.ncore_blocks[1] > 0) + 1;
   }
   HT_TRY(batch_pass(b, L, 2, st, count, x, dims, order, trees, cfg, U, B, want_err, eig_ctas));
-  HT_CUDA(cudaEventRecordWithFlags(b.tp[2], st, cudaEventRecordExternal));
+  HT_TRY(batch_phase_end(b, 2, st));
   HT_CUDA(transfer_tail_grouped_launch(static_cast<const TailJob *>(b.tails), L.ntail, st));
   b.launches += L.ntail > 0 ? 1 : 0;
-  HT_CUDA(cudaEventRecordWithFlags(b.tp[3], st, cudaEventRecordExternal));
+  HT_TRY(batch_phase_end(b, 3, st));
   if (L.nerr > 0) {
     const int *emaps[6];
     for (int k = 0; k < 6; ++k) emaps[k] = maps + L.map_off[2 + k];
@@ -2377,7 +2396,7 @@ ht_status_t batch_enqueue(BatchState &b, const BatchLayout &L, cudaStream_t st, 
     b.launches += 1;
   }
   HT_TRY(batch_pass(b, L, 3, st, count, x, dims, order, trees, cfg, U, B, want_err, eig_ctas));
-  HT_CUDA(cudaEventRecordWithFlags(b.tp[4], st, cudaEventRecordExternal));
+  HT_TRY(batch_phase_end(b, 4, st));
   HT_CUDA(copy_segments_launch(static_cast<const CopySeg *>(b.copies), L.ncopy, st));
   b.launches += L.ncopy > 0 ? 1 : 0;
   return HT_OK;
@@ -2479,7 +2498,7 @@ ht_status_t batch_plan_grouped(BatchState &b, BatchLayout &L, int count, const f
   L.ngram[0] = static_cast<int>(P.grams[0].size() / tc_gram_item_bytes());
   L.ngram[1] = static_cast<int>(P.grams[1].size() / tc_gram_item_bytes());
   P.grams[0].insert(P.grams[0].end(), P.grams[1].begin(), P.grams[1].end());
-  eig_grouped_order(P.table);
+  L.nwide = eig_grouped_order(P.table);
   L.nprob = static_cast<int>(P.table.size() / eig_grouped_entry_bytes());
   L.iters = P.iters;
   L.refine = P.refine;
@@ -2837,6 +2856,7 @@ ht_status_t ht_decompose_batched(int count, const float *const *x, const long *d
     }
   }
   const bool replay = b.exec && key == b.key;
+  bool direct = false;   // this call's launches are not a graph's
   if (!replay) {
     std::vector<Tree> T(count);
     BatchLayout L;
@@ -2883,13 +2903,21 @@ ht_status_t ht_decompose_batched(int count, const float *const *x, const long *d
     HT_CUDA(tc_prepare());   // one-time kernel attributes outside the capture
     HT_CUDA(eig_prepare());
     if (L.grouped) HT_TRY(batch_plan_grouped(b, L, count, x, dims, order, T, cfg, U, B, want_err));
-    // record the batch into a graph (captured from a private stream: the
-    // caller's may be the legacy stream); if capture is refused, run it directly
+    // run the batch, and while the GPU works on it record it into a graph for
+    // the next call (captured from a private stream: the caller's may be the
+    // legacy stream); if capture is refused there is none, and the reason is
+    // left in ht_last_error()
+    HT_CUDA(cudaEventRecord(b.t0, st));
+    HT_TRY(batch_enqueue(b, L, st, count, x, dims, order, T, cfg, U, B, want_err, eig_ctas));
+    HT_CUDA(cudaEventRecord(b.t1, st));
+    direct = true;
     bool captured = false;
     std::string why;
     cudaError_t ce = cudaStreamBeginCapture(b.cap, cudaStreamCaptureModeThreadLocal);
     if (ce == cudaSuccess) {
+      b.capturing = true;
       const ht_status_t s = batch_enqueue(b, L, b.cap, count, x, dims, order, T, cfg, U, B, want_err, eig_ctas);
+      b.capturing = false;
       if (s != HT_OK) why = ht_last_error();
       cudaGraph_t g = nullptr;
       ce = cudaStreamEndCapture(b.cap, &g);
@@ -2899,7 +2927,7 @@ ht_status_t ht_decompose_batched(int count, const float *const *x, const long *d
         b.graph = g;
         b.key = key;
         captured = true;
-      } else {   // not capturable here (or a launch failed): run the batch directly below
+      } else {   // not capturable here
         if (why.empty()) why = std::string("capture: ") + cudaGetErrorString(ce != cudaSuccess ? ce : ie);
         if (g) cudaGraphDestroy(g);
         b.exec = nullptr;
@@ -2910,16 +2938,6 @@ ht_status_t ht_decompose_batched(int count, const float *const *x, const long *d
       cudaGetLastError();
     }
     if (!captured) g_last_error = "batch ran without a CUDA graph (" + why + ")";
-    if (!captured) {
-      HT_CUDA(cudaEventRecord(b.t0, st));
-      HT_TRY(batch_enqueue(b, L, st, count, x, dims, order, T, cfg, U, B, want_err, eig_ctas));
-      HT_CUDA(cudaEventRecord(b.t1, st));
-    }
-    if (captured) {
-      HT_CUDA(cudaEventRecord(b.t0, st));
-      HT_CUDA(cudaGraphLaunch(b.exec, st));
-      HT_CUDA(cudaEventRecord(b.t1, st));
-    }
   } else {
     HT_CUDA(cudaEventRecord(b.t0, st));
     HT_CUDA(cudaGraphLaunch(b.exec, st));
@@ -2961,7 +2979,8 @@ ht_status_t ht_decompose_batched(int count, const float *const *x, const long *d
     report->lanes = b.lanes;
     report->grouped = b.grouped ? 1 : 0;
     if (b.grouped) {
-      const cudaEvent_t ev[7] = {b.t0, b.tp[0], b.tp[1], b.tp[2], b.tp[3], b.tp[4], b.t1};
+      const cudaEvent_t *tp = b.tp[direct ? 0 : 1];
+      const cudaEvent_t ev[7] = {b.t0, tp[0], tp[1], tp[2], tp[3], tp[4], b.t1};
       for (int i = 0; i < 6; ++i)
         if (cudaEventElapsedTime(&report->ms_phase[i], ev[i], ev[i + 1]) != cudaSuccess) {
           cudaGetLastError();   // timing unavailable: report zeros, leave no error behind

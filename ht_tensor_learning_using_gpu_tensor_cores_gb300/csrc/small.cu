@@ -169,25 +169,23 @@ __global__ void __launch_bounds__(256) convert_grouped_kernel(const ConvJob *__r
   load_job(jobs, job_of_block[blockIdx.x], J);
   const int b = blockIdx.x - J.blk0;
   Acc2 a = {0.f, 0.f};
-  // a warp per row of n1 inputs (n1p outputs), four loads in flight per lane
+  // a warp per eight rows of n1 inputs (n1p outputs), lanes along the rows: the
+  // eight loads of a lane are in flight together whatever the rows' length (a
+  // row at a time, 32 to 160 long, left most of four loads idle)
+  constexpr int RW = 8;
   const int lane = threadIdx.x & 31, n1 = static_cast<int>(J.n1), n1p = static_cast<int>(J.n1p);
-  for (long long r = static_cast<long long>(b) * 8 + (threadIdx.x >> 5); r < J.rest; r += J.nblk * 8ll) {
+  for (long long r = (static_cast<long long>(b) * 8 + (threadIdx.x >> 5)) * RW; r < J.rest; r += J.nblk * 8ll * RW) {
+    const int nr = static_cast<int>(min(static_cast<long long>(RW), J.rest - r));
     const float *src = J.x + J.n1 * r;
     __nv_bfloat16 *dst = J.xb ? J.xb + J.n1p * r : nullptr;
-    for (int i0 = lane; i0 < n1p; i0 += 128) {
-      float v[4];
+    for (int i = lane; i < n1p; i += 32) {
+      float v[RW];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + 32 * u;
-        v[u] = i < n1 ? __ldcs(src + i) : 0.f;
-      }
+      for (int u = 0; u < RW; ++u) v[u] = i < n1 && u < nr ? __ldcs(src + n1 * u + i) : 0.f;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + 32 * u;
-        if (i < n1p) {
-          acc2_add_prod(a, v[u], v[u]);
-          if (dst) dst[i] = __float2bfloat16_rn(v[u]);
-        }
+      for (int u = 0; u < RW; ++u) {
+        acc2_add_prod(a, v[u], v[u]);
+        if (dst && u < nr) dst[n1p * u + i] = __float2bfloat16_rn(v[u]);
       }
     }
   }
@@ -329,7 +327,10 @@ __global__ void __launch_bounds__(256) core_step2_kernel(const float *__restrict
 // Grouped narrow mode product of the batched path (the 3rd-order core pass,
 // rows of X contiguous): Z[row + L R j] = sum_i X[l + L (i + N r)] V[i + N j]
 // for row = l + L r, j < kz <= KB.  A thread per row, V staged in 64-row chunks
-// of shared memory; the job's blocks stride over its rows.
+// of shared memory; the job's blocks stride over its rows.  Fused operations in
+// pairs and the next eight loads in flight: 715 us to 633 over the 1.9 GB of 512
+// tensors of 32 to 160 a mode.  (Two rows a thread, as in the error pass, leave
+// too few warps for the loads: 734.)
 template <int KB>
 __global__ void __launch_bounds__(256) modeprod_narrow_grouped_kernel(const NarrowJob *__restrict__ jobs,
                                                                       const int *__restrict__ job_of_block) {
@@ -343,9 +344,9 @@ __global__ void __launch_bounds__(256) modeprod_narrow_grouped_kernel(const Narr
     const bool valid = row < total;
     const long long r = valid ? row / L : 0, l = valid ? row - r * L : 0;
     const float *x = J.X + l + L * N * r;
-    float acc[KB];
+    float2 acc[KB / 2];
 #pragma unroll
-    for (int j = 0; j < KB; ++j) acc[j] = 0.f;
+    for (int j = 0; j < KB / 2; ++j) acc[j] = make_float2(0.f, 0.f);
     for (int i0 = 0; i0 < N; i0 += 64) {
       const int ni = min(64, N - i0);
       __syncthreads();
@@ -355,20 +356,25 @@ __global__ void __launch_bounds__(256) modeprod_narrow_grouped_kernel(const Narr
       }
       __syncthreads();
       if (valid) {
-        for (int ii = 0; ii < ni; ii += 8) {
-          float xv[8];   // eight independent loads in flight before the products
+        // the next eight loads are in flight while the current eight are used
+        float xv[8], xn[8];
+        auto fetch = [&](int ii, float (&d)[8]) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) xv[u] = ii + u < ni ? __ldg(x + L * (i0 + ii + u)) : 0.f;
+          for (int u = 0; u < 8; ++u) d[u] = ii + u < ni ? __ldg(x + L * (i0 + ii + u)) : 0.f;
+        };
+        fetch(0, xn);
+        for (int ii = 0; ii < ni; ii += 8) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) xv[u] = xn[u];
+          fetch(ii + 8, xn);
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const float4 *v4 = reinterpret_cast<const float4 *>(&Vs[(ii + u) & 63][0]);
 #pragma unroll
             for (int j4 = 0; j4 < KB / 4; ++j4) {
               const float4 v = v4[j4];
-              acc[4 * j4] = fmaf(xv[u], v.x, acc[4 * j4]);
-              acc[4 * j4 + 1] = fmaf(xv[u], v.y, acc[4 * j4 + 1]);
-              acc[4 * j4 + 2] = fmaf(xv[u], v.z, acc[4 * j4 + 2]);
-              acc[4 * j4 + 3] = fmaf(xv[u], v.w, acc[4 * j4 + 3]);
+              fma2(acc[2 * j4], make_float2(xv[u], xv[u]), make_float2(v.x, v.y));
+              fma2(acc[2 * j4 + 1], make_float2(xv[u], xv[u]), make_float2(v.z, v.w));
             }
           }
         }
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(256) modeprod_narrow_grouped_kernel(const Narr
     if (valid)
 #pragma unroll
       for (int j = 0; j < KB; ++j)
-        if (j < kz) J.Z[row + total * j] = acc[j];
+        if (j < kz) J.Z[row + total * j] = j & 1 ? acc[j / 2].y : acc[j / 2].x;
   }
 }
 
@@ -651,55 +657,66 @@ __global__ void __launch_bounds__(256) err_expand2w_grouped_kernel(const ErrJob 
 // X[l + L i3] - sum_c W[l, c] U3[i3 + nc c] (U3 staged in 64-row chunks of
 // shared memory); the compensated sum of squares of a block's rows is its
 // partial (ntile = nblk[4] partials).
+// Two rows a thread, 256 apart, and rows of U_c in pairs: the broadcast loads of
+// U_c bound the kernel (930 us at one row a thread over the 1.9 GB of 512 tensors
+// of 32 to 160 a mode, 650 at two).
 template <int KB>
 __global__ void __launch_bounds__(256) err_narrow_grouped_kernel(const ErrJob *__restrict__ jobs,
                                                                  const int *__restrict__ job_of_block) {
   __shared__ ErrJob J;
-  __shared__ __align__(16) float Us[64][KB];
+  __shared__ __align__(16) float2 Us[32][KB];   // rows of U_c in pairs (2 p, 2 p + 1)
   __shared__ double red[256];
   load_job(jobs, job_of_block[blockIdx.x], J);
-  const int t = threadIdx.x, kc = J.kc, np = J.np, kq = J.kq;
+  const int t = threadIdx.x, kc = J.kc;
   const long long L = J.R, nc = J.Cn;
   const long long b = blockIdx.x - J.blk0[4];
   Acc2 acc = {0.f, 0.f};
-  for (long long base = b * 256; base < L; base += J.nblk[4] * 256ll) {
-    const long long l = base + t;
-    const bool valid = l < L;
-    const int i1 = valid ? static_cast<int>(l % np) : 0, i2 = valid ? static_cast<int>(l / np) : 0;
-    float w[KB];   // this row of the expansion (err_expand2w_grouped_kernel)
+  for (long long base = b * 512; base < L; base += J.nblk[4] * 512ll) {
+    float w[2][KB];   // the rows of the expansion (err_expand2w_grouped_kernel)
+    bool valid[2];
 #pragma unroll
-    for (int c = 0; c < KB; ++c) w[c] = (valid && c < kc) ? J.Wm[l + L * c] : 0.f;
+    for (int h = 0; h < 2; ++h) {
+      const long long l = base + t + 256 * h;
+      valid[h] = l < L;
+#pragma unroll
+      for (int c = 0; c < KB; ++c) w[h][c] = (valid[h] && c < kc) ? J.Wm[l + L * c] : 0.f;
+    }
+    const float *x = J.X + base + t;
     for (long long i0 = 0; i0 < nc; i0 += 64) {
       const int ni = static_cast<int>(min(64ll, nc - i0));
       __syncthreads();
       for (int e = t; e < 64 * KB; e += 256) {
-        const int ii = e / KB, c = e - ii * KB;
-        Us[ii][c] = (ii < ni && c < kc) ? J.B[(i0 + ii) + J.ldb * c] : 0.f;
+        const int c = e / 64, ii = e - c * 64;
+        reinterpret_cast<float *>(&Us[ii >> 1][c])[ii & 1] = (ii < ni && c < kc) ? J.B[(i0 + ii) + J.ldb * c] : 0.f;
       }
       __syncthreads();
-      if (valid)
-        for (int ii = 0; ii < ni; ii += 8) {
-          float xv[8];   // eight independent loads in flight before the products
+      for (int ii = 0; ii < ni; ii += 8) {
+        float xv[2][8];   // sixteen independent loads in flight before the products
 #pragma unroll
-          for (int u = 0; u < 8; ++u) xv[u] = ii + u < ni ? __ldcs(J.X + l + L * (i0 + ii + u)) : 0.f;
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            if (ii + u < ni) {
-              const float4 *u4 = reinterpret_cast<const float4 *>(&Us[ii + u][0]);
-              float xh = 0.f;
+          for (int u = 0; u < 8; ++u)
+            xv[h][u] = ii + u < ni && valid[h] ? __ldcs(x + 256 * h + L * (i0 + ii + u)) : 0.f;
 #pragma unroll
-              for (int c4 = 0; c4 < KB / 4; ++c4) {
-                const float4 v = u4[c4];
-                xh = fmaf(w[4 * c4], v.x, xh);
-                xh = fmaf(w[4 * c4 + 1], v.y, xh);
-                xh = fmaf(w[4 * c4 + 2], v.z, xh);
-                xh = fmaf(w[4 * c4 + 3], v.w, xh);
-              }
-              const float d = xv[u] - xh;
-              acc2_add_prod(acc, d, d);
+        for (int u = 0; u < 4; ++u) {
+          float2 xh[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+          for (int c = 0; c < KB; c += 2) {   // two columns of a pair of rows per load
+            const float4 v = *reinterpret_cast<const float4 *>(&Us[(ii >> 1) + u][c]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              fma2(xh[h], make_float2(w[h][c], w[h][c]), make_float2(v.x, v.y));
+              fma2(xh[h], make_float2(w[h][c + 1], w[h][c + 1]), make_float2(v.z, v.w));
             }
           }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {   // (rows past the edges: x, w and u are zero)
+            const float d0 = xv[h][2 * u] - xh[h].x, d1 = xv[h][2 * u + 1] - xh[h].y;
+            acc2_add_prod(acc, d0, d0);
+            acc2_add_prod(acc, d1, d1);
+          }
         }
+      }
     }
   }
   red[t] = static_cast<double>(acc.s) + static_cast<double>(acc.c);

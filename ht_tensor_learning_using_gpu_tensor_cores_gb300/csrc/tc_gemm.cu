@@ -392,7 +392,9 @@ bool tc_gram_item(const Operand &a, long n, float *G, int *err, std::vector<unsi
   GramItem it;
   std::memset(&it, 0, sizeof(it));
   const int bmt = cls == 0 ? BM : 2 * BM, bn = cls == 0 ? BM : 2 * BM;
-  if (!make_map(a, bmt, &it.map_a, why) || !make_map(a, bn, &it.map_b, why)) return false;
+  if (!make_map(a, bmt, &it.map_a, why)) return false;
+  it.map_b = it.map_a;   // both operands' boxes have the same rows
+  static_assert(sizeof(it.map_a) == sizeof(it.map_b), "one map");
   KParams &p = it.p;
   p.a_kind = p.b_kind = a.kind;
   p.a_lblocks = p.b_lblocks = int((a.d0 + BK - 1) / BK);
