@@ -3312,6 +3312,7 @@ ht_status_t ht_evaluate(const long *dims, int order, const ht_tree_t *tree, cons
   //   W12[i0][r1 + k1 b] = sum_a U_a1[i0, a] B_t1[a, b, r1]
   //   W34[i2][r1 + k1 d] = sum_{c, r2} U_a2[i2, c] B_t2[c, d, r2] B_root[r1, r2]
   //   entry = sum_r1 (sum_b W12[i0][r1, b] U_b1[i1, b]) (sum_d W34[i2][r1, d] U_b2[i3, d]).
+  bool grouped = true;
   auto plan = [&](Ctx &c) -> ht_status_t {
     const float *Ud[HT_MAX_NODES] = {}, *Bd[HT_MAX_NODES] = {};
     c.err = c.ar.take<int>(64);
@@ -3371,20 +3372,44 @@ ht_status_t ht_evaluate(const long *dims, int order, const ht_tree_t *tree, cons
       ep.side[0] = EvalSide{W12, Ud[b1], dims[0], dims[1], 0, 1, kb1};
       ep.side[1] = EvalSide{W34, Ud[b2], dims[2], dims[3], 2, 3, kb2};
     }
+    const bool group = grouped && evaluate_groups(ep, count);
+    EvalGroups g{};
+    if (group) {
+      const EvalSide &S0 = ep.side[0], &S1 = ep.side[1];
+      g.Uq = c.ar.take<float>(static_cast<size_t>(S0.n_vec) * ((S0.kx + 3) / 4 * 4));
+      g.Uc = c.ar.take<float>(static_cast<size_t>(S1.n_vec) * ((ep.ky + 3) / 4 * 4));
+      g.hist = c.ar.take<int>(static_cast<size_t>(2 * S0.n_row));
+      g.rec = c.ar.take<int4>(static_cast<size_t>(std::min(count, kEvalChunk)));
+      if (!g.Uq || !g.Uc || !g.hist || !g.rec) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small");
+    }
     if (!c.dry()) {
       HT_CUDA(cudaMemsetAsync(c.err, 0, sizeof(int), c.st));
-      HT_CUDA(evaluate_launch(ep, ix, count, o, c.err, c.st));
-      ++c.launches;
+      if (group) {
+        HT_CUDA(evaluate_grouped_launch(ep, g, ix, count, o, c.err, c.st, &c.launches));
+      } else {
+        HT_CUDA(evaluate_launch(ep, ix, count, o, c.err, c.st));
+        ++c.launches;
+      }
       if (!out_dev) HT_CUDA(cudaMemcpyAsync(out, o, sizeof(float) * count, cudaMemcpyDeviceToHost, c.st));
     }
     return HT_OK;
   };
-  Ctx d;
-  d.ar.dry = true;
-  HT_TRY(plan(d));
-  const size_t bytes = d.ar.peak + (1 << 20);
   void *ws = nullptr;
-  HT_TRY(acquire_workspace(bytes, &ws, st));
+  size_t bytes = 0;
+  auto acquire = [&]() -> ht_status_t {
+    Ctx d;
+    d.ar.dry = true;
+    HT_TRY(plan(d));
+    bytes = d.ar.peak + (1 << 20);
+    return acquire_workspace(bytes, &ws, st);
+  };
+  ht_status_t got = acquire();
+  if (got == HT_ERR_OUT_OF_MEMORY) {   // no room for the records: entry by entry
+    cudaGetLastError();
+    grouped = false;
+    got = acquire();
+  }
+  HT_TRY(got);
   Ctx c;
   c.st = st;
   c.ar.base = static_cast<char *>(ws);

@@ -436,6 +436,19 @@ struct EvalPlan {
 // an index out of range sets *err to 1.
 cudaError_t evaluate_launch(const EvalPlan &ep, const long long *idx, long long count, float *out, int *err,
                             cudaStream_t s);
+// The same for many entries whose second side has no W, grouped by the row of W
+// (a path of its own where evaluate_groups says so).
+struct EvalGroups {
+  float *Uq, *Uc;   // both sides' Uv, rows contiguous: n_vec x (kx, ky rounded up to a multiple of 4)
+  int *hist;        // [2 n_row]
+  int4 *rec;        // [min(count, kEvalChunk)]
+};
+constexpr long long kEvalChunk = 1 << 22;   // entries sorted at a time: 64 MB of records stay in L2
+constexpr int kEvalGroupRows = 6000;        // rows of W counted in 48 KB of shared memory (two integers each)
+constexpr long long kEvalGroupMin = 3000000;
+bool evaluate_groups(const EvalPlan &ep, long long count);
+cudaError_t evaluate_grouped_launch(const EvalPlan &ep, const EvalGroups &g, const long long *idx, long long count,
+                                    float *out, int *err, cudaStream_t s, int *launches);
 
 // ------------------------------------------------------ HT tensor layer (layer.cu)
 constexpr int kLayerMaxRank = 64;

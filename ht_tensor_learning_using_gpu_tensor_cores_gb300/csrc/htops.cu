@@ -9,6 +9,8 @@
 // precontracted matrices: every transfer tensor is folded with its parent's
 // and one child's factors into a matrix with one row per index of that child's
 // mode, so an entry costs one or two k x k row-vector products.
+#include <climits>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -144,6 +146,283 @@ __global__ void __launch_bounds__(256) evaluate_kernel(const EvalPlan ep, const 
   }
 }
 
+// Many entries of a 3rd-order tensor.  The warp above reads its entry's whole row
+// of W (4 KB at rank 32) from L2, which bounds it.  Here the entries are first
+// grouped by that row (a counting sort of 16-byte records), so that a block
+// stages a row once for all its entries, and a thread forms several entries at
+// once from it.
+constexpr int kEvalThreads = 128, kEvalPer = 2;   // threads, entries a thread
+constexpr int kSortThreads = 1024, kSortEntries = 8 * kSortThreads;   // entries per sorting block
+
+HT_DEV void cp_async16(void *smem_dst, const void *gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+}
+HT_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+HT_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The leaf bases (n x k, mode-major) with their rows contiguous, padded to a
+// multiple of four columns: an entry's row is a few 16-byte loads instead of k
+// scattered ones.  Blocks below blocks0 take the first basis.
+__global__ void __launch_bounds__(256) eval_rows_kernel(const float *__restrict__ A0, long long n0, int k0,
+                                                        float *__restrict__ R0, int blocks0,
+                                                        const float *__restrict__ A1, long long n1, int k1,
+                                                        float *__restrict__ R1) {
+  __shared__ float tile[32][65];
+  const bool second = static_cast<int>(blockIdx.x) >= blocks0;
+  const float *A = second ? A1 : A0;
+  float *R = second ? R1 : R0;
+  const long long n = second ? n1 : n0;
+  const int k = second ? k1 : k0, kr = (k + 3) / 4 * 4;
+  const long long r0 = 32ll * (blockIdx.x - (second ? blocks0 : 0));
+  const int nr = static_cast<int>(min(32ll, n - r0));
+  for (int e = threadIdx.x; e < 32 * kr; e += 256) {
+    const int r = e & 31, c = e >> 5;
+    tile[r][c] = r < nr && c < k ? A[r0 + r + n * c] : 0.f;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < nr * kr; e += 256) R[r0 * kr + e] = tile[e / kr][e % kr];
+}
+
+// Entries per row of W.
+__global__ void __launch_bounds__(kSortThreads) eval_count_kernel(const long long *__restrict__ idx, int count,
+                                                                  int order, int mode, int n, int *__restrict__ hist) {
+  extern __shared__ int sh[];
+  for (int i = threadIdx.x; i < n; i += kSortThreads) sh[i] = 0;
+  __syncthreads();
+  const long long e0 = static_cast<long long>(blockIdx.x) * kSortEntries;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const long long e = e0 + u * kSortThreads + threadIdx.x;
+    if (e < count) {
+      const long long i = idx[e * order + mode];
+      atomicAdd(&sh[i < 0 ? 0 : i >= n ? n - 1 : static_cast<int>(i)], 1);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += kSortThreads)
+    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+}
+
+// Records (row of U_q, row of U_c, entry, row of W) in order of the row of W.
+// Every block sums the counts (n integers), takes room for its own entries of
+// each row with one atomic per row and writes them there: the order within a
+// row is the blocks' and plays no part in an entry's value.
+__global__ void __launch_bounds__(kSortThreads) eval_sort_kernel(const EvalPlan ep, const long long *__restrict__ idx,
+                                                                 int count, const int *__restrict__ hist,
+                                                                 int *__restrict__ taken, int4 *__restrict__ rec,
+                                                                 int *err) {
+  extern __shared__ int sh[];   // first[n], mine[n]
+  __shared__ int wsum[32];
+  const EvalSide &S0 = ep.side[0], &S1 = ep.side[1];
+  const int n = static_cast<int>(S0.n_row), t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int *first = sh, *mine = sh + n;
+  const int per = (n + kSortThreads - 1) / kSortThreads, lo = min(n, t * per), hi = min(n, lo + per);
+  int sum = 0;
+  for (int i = lo; i < hi; ++i) {
+    sum += hist[i];
+    mine[i] = 0;
+  }
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) wsum[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    int w = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += v;
+    }
+    wsum[lane] = w;
+  }
+  __syncthreads();
+  int at = inc - sum + (warp ? wsum[warp - 1] : 0);
+  for (int i = lo; i < hi; ++i) {
+    first[i] = at;
+    at += hist[i];
+  }
+  __syncthreads();
+  const long long e0 = static_cast<long long>(blockIdx.x) * kSortEntries;
+  int4 r[8];
+  int rank[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const long long e = e0 + u * kSortThreads + t;
+    rank[u] = -1;
+    if (e < count) {
+      r[u].x = static_cast<int>(eval_index(idx, e, ep.order, S0.mode_vec, S0.n_vec, err, 0));
+      r[u].y = static_cast<int>(eval_index(idx, e, ep.order, S1.mode_vec, S1.n_vec, err, 0));
+      r[u].z = static_cast<int>(e);
+      r[u].w = static_cast<int>(eval_index(idx, e, ep.order, S0.mode_row, S0.n_row, err, 0));
+      rank[u] = atomicAdd(&mine[r[u].w], 1);
+    }
+  }
+  __syncthreads();
+  for (int i = t; i < n; i += kSortThreads)
+    if (mine[i]) first[i] += atomicAdd(&taken[i], mine[i]);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (rank[u] >= 0) rec[first[r[u].w] + rank[u]] = r[u];
+}
+
+// A thread holds two entries' ky <= KB sums over x as packed pairs, so that a
+// row's values, broadcast from shared memory, serve two entries each (four
+// entries halve those loads but leave eight warps an SM where these two have
+// sixteen: 239 us a call against 194 at 1048576 entries, 1024 rows, rank 32).
+// A block takes 256 records and stages each row of W that they use in turn; a
+// warp fetches the basis rows of its 64 entries with whole-row copies into
+// shared memory at an odd pitch of 16 bytes (each thread loading its own rows
+// touches 32 lines an instruction).  Entry by entry the call took 881 us.
+template <int KB>
+__global__ void __launch_bounds__(kEvalThreads) evaluate_grouped_kernel(const EvalPlan ep, const EvalGroups g, int count,
+                                                                        float *__restrict__ out) {
+  extern __shared__ __align__(16) float4 eval_rows[];   // [warps][32 kEvalPer][pitch]
+  __shared__ __align__(16) float Ps[KB][KB];            // [x][y]
+  __shared__ int2 row_of[kEvalThreads * kEvalPer];
+  __shared__ int last_key[kEvalThreads / 32], runs[kEvalThreads / 32], run_key[kEvalThreads * kEvalPer];
+  const int t = threadIdx.x, lane = t & 31, kx = ep.side[0].kx, ky = ep.ky;
+  const int lq = (kx + 3) / 4, lc = (ky + 3) / 4, pitch = KB / 4 + 1;
+  const int base = blockIdx.x * (kEvalThreads * kEvalPer), end = min(count, base + kEvalThreads * kEvalPer);
+  float4 *rows = eval_rows + (t >> 5) * (32 * kEvalPer * pitch);
+  int2 *ids = row_of + (t & ~31) * kEvalPer;
+  int key[kEvalPer], dst[kEvalPer];
+#pragma unroll
+  for (int u = 0; u < kEvalPer; ++u) {
+    const int e = base + (t & ~31) * kEvalPer + 32 * u + lane;
+    const int4 r = e < end ? g.rec[e] : make_int4(0, 0, 0, -1);
+    ids[32 * u + lane] = make_int2(r.x, r.y);
+    dst[u] = r.z;
+    key[u] = r.w;
+  }
+  // the block's distinct rows of W in order (its records are sorted by them)
+  const int warp = t >> 5;
+  if (lane == 31) last_key[warp] = key[kEvalPer - 1];
+  __syncthreads();
+  int before = warp ? last_key[warp - 1] : -1, nrun = 0;
+  unsigned heads[kEvalPer];
+#pragma unroll
+  for (int u = 0; u < kEvalPer; ++u) {
+    int prev = __shfl_up_sync(0xffffffffu, key[u], 1);
+    if (lane == 0) prev = before;
+    before = __shfl_sync(0xffffffffu, key[u], 31);
+    heads[u] = __ballot_sync(0xffffffffu, key[u] >= 0 && key[u] != prev);
+    nrun += __popc(heads[u]);
+  }
+  if (lane == 0) runs[warp] = nrun;
+  __syncthreads();
+  int at = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kEvalThreads / 32; ++w) {
+    at += w < warp ? runs[w] : 0;
+    total += runs[w];
+  }
+#pragma unroll
+  for (int u = 0; u < kEvalPer; ++u) {
+    if ((heads[u] >> lane) & 1u) run_key[at + __popc(heads[u] & ((1u << lane) - 1u))] = key[u];
+    at += __popc(heads[u]);
+  }
+  __syncthreads();
+  // rows of U (l 16-byte pieces each) of this warp's entries
+  auto fetch = [&](const float *U, int l, bool second) {
+    const int dr = 32 / l, dc = 32 - dr * l;
+    int r = lane / l, c = lane - r * l;
+    while (r < 32 * kEvalPer) {
+      const int row = second ? ids[r].y : ids[r].x;
+      cp_async16(rows + r * pitch + c, reinterpret_cast<const float4 *>(U) + static_cast<long long>(row) * l + c);
+      r += dr;
+      c += dc;
+      if (c >= l) {
+        c -= l;
+        ++r;
+      }
+    }
+    cp_async_commit();
+  };
+  for (int run = 0; run < total; ++run) {
+    const int cur = run_key[run];
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < kEvalPer; ++u) any = any || key[u] == cur;
+    any = __any_sync(0xffffffffu, any);
+    if (any) fetch(g.Uq, lq, false);
+    __syncthreads();
+    const float *W = ep.side[0].W + static_cast<long long>(cur) * ky * kx;
+    for (int e = t; e < 4 * lq * KB; e += kEvalThreads) {
+      const int x = e / KB, y = e - x * KB;
+      Ps[x][y] = x < kx && y < ky ? W[y + ky * x] : 0.f;
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    if (any) {
+      float2 acc[kEvalPer][KB / 2];
+#pragma unroll
+      for (int u = 0; u < kEvalPer; ++u)
+#pragma unroll
+        for (int y = 0; y < KB / 2; ++y) acc[u][y] = make_float2(0.f, 0.f);
+#pragma unroll 1
+      for (int x = 0; x < lq; ++x) {
+        float4 q[kEvalPer];
+#pragma unroll
+        for (int u = 0; u < kEvalPer; ++u) q[u] = rows[(32 * u + lane) * pitch + x];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+#pragma unroll
+          for (int y = 0; y < KB; y += 4) {
+            const float4 p = *reinterpret_cast<const float4 *>(&Ps[4 * x + v][y]);
+#pragma unroll
+            for (int u = 0; u < kEvalPer; ++u) {
+              const float w = v == 0 ? q[u].x : v == 1 ? q[u].y : v == 2 ? q[u].z : q[u].w;
+              fma2(acc[u][y / 2], make_float2(w, w), make_float2(p.x, p.y));
+              fma2(acc[u][y / 2 + 1], make_float2(w, w), make_float2(p.z, p.w));
+            }
+          }
+        }
+      }
+      __syncwarp();
+      fetch(g.Uc, lc, true);
+      cp_async_wait_all();
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < kEvalPer; ++u) {
+        float part[KB / 4];   // (columns past ky take no part: 0 times infinity)
+#pragma unroll
+        for (int y = 0; y < KB; y += 4) {
+          part[y / 4] = 0.f;
+          if (y < ky) {
+            const float4 c = rows[(32 * u + lane) * pitch + (y >> 2)];
+            const float2 a = acc[u][y / 2], b = acc[u][y / 2 + 1];
+            const float lo = y + 1 < ky ? fmaf(a.y, c.y, a.x * c.x) : a.x * c.x;
+            const float hi = y + 2 < ky ? (y + 3 < ky ? fmaf(b.y, c.w, b.x * c.z) : b.x * c.z) : 0.f;
+            part[y / 4] = lo + hi;
+          }
+        }
+#pragma unroll
+        for (int w = 1; w < KB / 4; w *= 2)
+#pragma unroll
+          for (int y = 0; y + w < KB / 4; y += 2 * w) part[y] += part[y + w];
+        if (key[u] == cur) out[dst[u]] = part[0];
+      }
+      __syncwarp();
+    }
+  }
+}
+
+template <int KB>
+cudaError_t evaluate_grouped_kb(const EvalPlan &ep, const EvalGroups &g, int count, float *out, cudaStream_t s) {
+  constexpr int smem = kEvalThreads * kEvalPer * (KB / 4 + 1) * 16;
+  const cudaError_t e = cudaFuncSetAttribute(evaluate_grouped_kernel<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             smem);
+  if (e != cudaSuccess) return e;
+  const unsigned grid = static_cast<unsigned>((count + kEvalThreads * kEvalPer - 1) / (kEvalThreads * kEvalPer));
+  evaluate_grouped_kernel<KB><<<grid, kEvalThreads, smem, s>>>(ep, g, count, out);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t gemm_nt_launch(const float *A, long long lda, long long sA, const float *B, long long ldb, float *C,
@@ -182,6 +461,47 @@ cudaError_t evaluate_launch(const EvalPlan &ep, const long long *idx, long long 
   if (grid < 1) grid = 1;
   evaluate_kernel<<<static_cast<unsigned>(grid), 256, 0, s>>>(ep, idx, count, out, err);
   return cudaGetLastError();
+}
+
+// Grouping pays from some count on.  Entry by entry costs ~0.02 ns (kx + 8) an
+// entry (1048576 entries at 400^3: 345, 552, 879 us for a whole call at ranks 6,
+// 16, 32); grouped, the same take 140, 150, 200 with ~40 us of sorting launches,
+// which 65536 entries do not earn back at rank 32 (139 against 156) and just do
+// at rank 40 (151 against 144).  With few entries a row the blocks mostly wait
+// for the next row: 262144 entries of 1400 rows still gain (299 to 210 at rank
+// 32), 65536 lose (143 to 225).
+bool evaluate_groups(const EvalPlan &ep, long long count) {
+  const EvalSide &S0 = ep.side[0], &S1 = ep.side[1];
+  return S0.W && !S1.W && S0.kx <= 64 && ep.ky <= 64 && S0.n_row <= kEvalGroupRows && S0.n_vec <= INT_MAX &&
+         S1.n_vec <= INT_MAX && count >= 128 * S0.n_row && count * (S0.kx + 8) >= kEvalGroupMin;
+}
+
+cudaError_t evaluate_grouped_launch(const EvalPlan &ep, const EvalGroups &g, const long long *idx, long long count,
+                                    float *out, int *err, cudaStream_t s, int *launches) {
+  const EvalSide &S0 = ep.side[0], &S1 = ep.side[1];
+  const int n = static_cast<int>(S0.n_row);
+  const long long b0 = (S0.n_vec + 31) / 32, b1 = (S1.n_vec + 31) / 32;
+  if (b0 + b1 > INT_MAX) return cudaErrorInvalidValue;
+  eval_rows_kernel<<<static_cast<unsigned>(b0 + b1), 256, 0, s>>>(S0.Uv, S0.n_vec, S0.kx, g.Uq, static_cast<int>(b0),
+                                                                  S1.Uv, S1.n_vec, ep.ky, g.Uc);
+  ++*launches;
+  for (long long e0 = 0; e0 < count; e0 += kEvalChunk) {
+    const int cn = static_cast<int>(count - e0 < kEvalChunk ? count - e0 : kEvalChunk);
+    const unsigned blocks = static_cast<unsigned>((cn + kSortEntries - 1) / kSortEntries);
+    cudaError_t e = cudaMemsetAsync(g.hist, 0, 2 * sizeof(int) * n, s);   // hist, taken
+    if (e != cudaSuccess) return e;
+    const long long *ix = idx + e0 * ep.order;
+    eval_count_kernel<<<blocks, kSortThreads, n * sizeof(int), s>>>(ix, cn, ep.order, S0.mode_row, n, g.hist);
+    eval_sort_kernel<<<blocks, kSortThreads, 2 * n * sizeof(int), s>>>(ep, ix, cn, g.hist, g.hist + n, g.rec, err);
+    const int k = ep.ky > S0.kx ? ep.ky : S0.kx;
+    e = k <= 16   ? evaluate_grouped_kb<16>(ep, g, cn, out + e0, s)
+        : k <= 32 ? evaluate_grouped_kb<32>(ep, g, cn, out + e0, s)
+        : k <= 48 ? evaluate_grouped_kb<48>(ep, g, cn, out + e0, s)
+                  : evaluate_grouped_kb<64>(ep, g, cn, out + e0, s);
+    if (e != cudaSuccess) return e;
+    *launches += 3;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace htgb
