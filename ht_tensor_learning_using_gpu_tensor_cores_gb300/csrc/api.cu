@@ -1065,26 +1065,29 @@ ht_status_t leaf_sketch(Ctx &c, const Tree &T, const ht_config_t &cfg, const lon
   }
   for (int m = 0; m < order; ++m) HT_TRY(apply_gram(m, Qm[m], Ym[m]));
   // Nystrom: W = Q^T Y, Y_nu = Y + nu Q -> Q1 R1, H = R1 (W + nu I)^-1 R1^T, U = Q1 * top-K(H)
+  GemmTnProb tn[4];
+  NystromShift shift[4];
   for (int m = 0; m < order; ++m) {
     const int n = static_cast<int>(dims[m]), s = S[m];
-    HT_CUDA(gemm_tn_small_launch(Qm[m], n, Ym[m], n, Wm[m], s, s, s, n, c.st));
-    HT_CUDA(nystrom_shift_launch(Ym[m], Qm[m], n, s, Wm[m], kNystromShift, Q1[m], c.st));
-    HT_CUDA(cudaMemcpyAsync(Ym[m], Q1[m], sizeof(float) * n * s, cudaMemcpyDeviceToDevice, c.st));   // Y_nu
-    c.launches += 2;
+    tn[m] = GemmTnProb{Qm[m], Ym[m], Wm[m], n, n, s, s, s, n};
+    shift[m] = NystromShift{Ym[m], Qm[m], Wm[m], Q1[m], n, s};
   }
+  HT_CUDA(gemm_tn_small_batched_launch(tn, order, c.st));
+  HT_CUDA(nystrom_shift_launch(shift, order, kNystromShift, c.st));   // Ym is Y_nu from here on
+  c.launches += 2;
   HT_TRY(orth_all(Q1));
   NystromProb np_[4];
   SvdGramProb sp[4];
   for (int m = 0; m < order; ++m) {
     const int n = static_cast<int>(dims[m]), s = S[m];
-    HT_CUDA(gemm_tn_small_launch(Q1[m], n, Ym[m], n, R1[m], s, s, s, n, c.st));
-    ++c.launches;
+    tn[m] = GemmTnProb{Q1[m], Ym[m], R1[m], n, n, s, s, s, n};
     np_[m] = NystromProb{Wm[m], R1[m], s, Hm[m]};
     sp[m] = SvdGramProb{Hm[m], s, K[m], K[m], Tm[m], M2[m], Br[m]};
   }
+  HT_CUDA(gemm_tn_small_batched_launch(tn, order, c.st));
   HT_CUDA(nystrom_core_launch(np_, order, kNystromShift, c.err, c.st));       // all modes, a CTA each
   HT_CUDA(svd_from_gram_batched_launch(sp, order, c.st));                     // top-K eigenvectors of each H
-  c.launches += 2;
+  c.launches += 3;
   for (int m = 0; m < order; ++m) {
     const int n = static_cast<int>(dims[m]), s = S[m];
     HT_CUDA(matmul_nn_launch(Q1[m], n, Tm[m], s, ep[m].U, n, n, K[m], s, c.st));

@@ -291,6 +291,13 @@ cudaError_t copy_segments_launch(const CopySeg *segs_dev, int nseg, cudaStream_t
 // C (m x n) = A^T B with A (K x m), B (K x n), column-major, compensated FP32.
 cudaError_t gemm_tn_small_launch(const float *A, int lda, const float *B, int ldb, float *C, int ldc, int m, int n,
                                  int K, cudaStream_t s);
+// The same for up to four problems in one launch.
+struct GemmTnProb {
+  const float *A, *B;
+  float *C;
+  int lda, ldb, ldc, m, n, K;
+};
+cudaError_t gemm_tn_small_batched_launch(const GemmTnProb *probs, int nprob, cudaStream_t s);
 // C[a + kp*b + kp*kq*c] = sum_j T1[(j + nq*c) + ldt*a] * Uq[j + nq*b].  scratch (or
 // null: one CTA per c) holds core_step2_ranges(nq, kc) * kp*kq*kc floats of partial
 // sums over ranges of j, summed in order afterwards.
@@ -390,9 +397,16 @@ cudaError_t tsqr_launch(const float *A, long long m, int k, long long lda, float
                         size_t ws_bytes, cudaStream_t st, int *launches);
 
 // ------------------------------------------- Gram-free leaf range finder (sketch.cu)
-// Yn = Y + nu Q (n x s), nu = nu_rel * tr(W) for the s x s matrix W.
-cudaError_t nystrom_shift_launch(const float *Y, const float *Q, long long n, int s, const float *W, float nu_rel,
-                                 float *Yn, cudaStream_t st);
+// Y += nu Q (n x s), nu = nu_rel * tr(W) for the s x s matrix W, and a copy in
+// Yn (up to four problems in one launch).
+struct NystromShift {
+  float *Y;
+  const float *Q, *W;
+  float *Yn;
+  long long n;
+  int s;
+};
+cudaError_t nystrom_shift_launch(const NystromShift *probs, int nprob, float nu_rel, cudaStream_t st);
 // H (s x s) = R1 (sym(W) + nu I)^-1 R1^T, nu as above (FP64, one CTA per
 // problem; up to four problems in one launch).
 struct NystromProb {

@@ -6,6 +6,8 @@
 //   * expansion of HT factors and a fused reconstruct-and-reduce error pass
 //     that never materialises Xhat (the reference writes Xhat and runs
 //     Saxpy + 2 x Snrm2, htd_batch.cu:196-244).
+#include <algorithm>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -264,8 +266,15 @@ __global__ void sumsq_finish_kernel(const double *partials, int n, double *out) 
 
 // C (m x n) = A^T B, A (K x m), B (K x n), column-major.  One warp per output
 // element, compensated accumulation.
-__global__ void gemm_tn_small_kernel(const float *__restrict__ A, int lda, const float *__restrict__ B, int ldb,
-                                     float *__restrict__ C, int ldc, int m, int n, int K) {
+struct GemmTnBatch {
+  GemmTnProb p[4];
+};
+
+__global__ void gemm_tn_small_kernel(const GemmTnBatch batch) {
+  const GemmTnProb &p = batch.p[blockIdx.y];
+  const float *__restrict__ A = p.A, *__restrict__ B = p.B;
+  float *__restrict__ C = p.C;
+  const int lda = p.lda, ldb = p.ldb, ldc = p.ldc, m = p.m, n = p.n, K = p.K;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= m * n) return;
@@ -863,12 +872,22 @@ cudaError_t sumsq_finish_launch(const double *partials, int n, double *out, cuda
   return cudaGetLastError();
 }
 
+cudaError_t gemm_tn_small_batched_launch(const GemmTnProb *probs, int nprob, cudaStream_t s) {
+  if (nprob < 1 || nprob > 4) return cudaErrorInvalidValue;
+  GemmTnBatch b{};
+  long long warps = 1;
+  for (int i = 0; i < nprob; ++i) {
+    b.p[i] = probs[i];
+    warps = std::max(warps, static_cast<long long>(probs[i].m) * probs[i].n);
+  }
+  gemm_tn_small_kernel<<<dim3(static_cast<unsigned>((warps * 32 + 255) / 256), nprob), 256, 0, s>>>(b);
+  return cudaGetLastError();
+}
+
 cudaError_t gemm_tn_small_launch(const float *A, int lda, const float *B, int ldb, float *C, int ldc, int m, int n,
                                  int K, cudaStream_t s) {
-  const long long warps = static_cast<long long>(m) * n;
-  const int blocks = static_cast<int>((warps * 32 + 255) / 256);
-  gemm_tn_small_kernel<<<blocks, 256, 0, s>>>(A, lda, B, ldb, C, ldc, m, n, K);
-  return cudaGetLastError();
+  const GemmTnProb p{A, B, C, lda, ldb, ldc, m, n, K};
+  return gemm_tn_small_batched_launch(&p, 1, s);
 }
 
 int core_step2_ranges(int nq, int kc) {

@@ -19,6 +19,8 @@
 //     waits for another, so the launch needs no co-residency.
 // The result has a non-negative diagonal (R's rows take the sign of their
 // pivot); optionally R^T R is formed in compensated FP32.
+#include <cfloat>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -46,20 +48,23 @@ HT_DEV float warp_sum_bcast(float v) {
   return __shfl_sync(0xffffffffu, v, 0);
 }
 
-// Sum of v[i] over the warp for 32 columns i at once (reduce-scatter): lane l
-// returns the total of column l.  31 shuffles, all independent per level.
-HT_DEV float warp_reduce_scatter32(float (&v)[32]) {
+// Sum of v[i] over the warp for W (16 or 32) columns i at once (reduce-scatter):
+// lane l returns the total of column l (W = 32) or l / 2 (W = 16).  W - 1 or W
+// shuffles, all independent per level.
+template <int W>
+HT_DEV float warp_reduce_scatter(float (&v)[W]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
+  for (int o = 16, n = W / 2; n >= 1; o >>= 1, n >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const float send = up ? v[i] : v[i + o];
-      const float keep = up ? v[i + o] : v[i];
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n];
+      const float keep = up ? v[i + n] : v[i];
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
+  if (W == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
   return v[0];
 }
 
@@ -102,7 +107,7 @@ HT_DEV void warp_qr_fold(float *R, float *P, int prow, int k) {
           v[i] = fmaf(x0, a0[i], x1 * a1[i]);
         }
         const int cl = 32 * b + lane;        // this lane's column
-        const float w = fmaf(v0, r[b], warp_reduce_scatter32(v));
+        const float w = fmaf(v0, r[b], warp_reduce_scatter<32>(v));
         const float tw = (cl > j && cl < k) ? tau * w : 0.f;
         r[b] = fmaf(-tw, v0, r[b]);
 #pragma unroll
@@ -125,71 +130,86 @@ HT_DEV void warp_qr_fold(float *R, float *P, int prow, int k) {
 }
 
 // The same fold for k <= 32 with the panel in registers: lane l holds rows
-// l + 32 q (q < RPL) of all 32 columns.  The column extraction is a select over
-// the unrolled register array; the shuffles of one column step (the column
-// norm, the 32-column reduce-scatter and the broadcast of the 32 updates) are
-// shared by all 32 RPL rows of the panel, so taller panels amortise them.
-template <int LD, int RPL>
-HT_DEV void warp_qr_fold32(float *R, float (&p)[RPL][32], int k) {
-  const int lane = threadIdx.x & 31;
-  for (int j = 0; j < k; ++j) {
-    float r = lane < k ? R[j * LD + lane] : 0.f;
-    float x[RPL];
+// l + 32 q in packed pairs of q.  The fold is one dependent chain per column (a
+// CTA of the tall case runs 15 folds of 32 columns in a row), so a column is
+// kept short: the current column is always index 0 (the update writes column c
+// to c - 1, no look-up by j), its norm is the reflector's dot product with
+// itself from the same reduce-scatter as the others', the updates' factors are
+// shared through W floats of shared memory, and once at most 16 columns are
+// left the steps take only those.  261 us to 101 for 409600 rows of 32.
+template <int W, int LD, int Q2>
+HT_DEV void warp_qr_columns(float *R, float2 (&p)[Q2][32], int j0, int j1, int k, float *fac) {
+  const int lane = threadIdx.x & 31, cl = W == 32 ? lane : lane >> 1;   // this lane's column, from j on
+  for (int j = j0; j < j1; ++j) {
+    const bool live = j + cl < k;
+    float r = live ? R[j * LD + j + cl] : 0.f;
+    float2 x[Q2];
 #pragma unroll
-    for (int q = 0; q < RPL; ++q) {
-      x[q] = 0.f;
+    for (int q = 0; q < Q2; ++q) x[q] = p[q][0];
+    float v[W];
 #pragma unroll
-      for (int c = 0; c < 32; ++c)
-        if (c == j) x[q] = p[q][c];
+    for (int c = 0; c < W; ++c) {
+      float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < Q2; ++q) fma2(a, x[q], p[q][c]);
+      v[c] = a.x + a.y;
     }
-    float ss = 0.f;
+    const float dot = warp_reduce_scatter<W>(v);
+    const float sig = __shfl_sync(0xffffffffu, dot, 0), rjj = __shfl_sync(0xffffffffu, r, 0);
+    const float nrm = sqrtf(fmaf(rjj, rjj, sig));
+    const float alpha = rjj > 0.f ? -nrm : nrm;
+    const float v0 = rjj - alpha, av = alpha * v0;   // reflector v = [v0; x], tau = 2 / v^T v = -1 / av
+    float tw = 0.f;
+    // otherwise the column below the pivot is zero, or what rounding left of a
+    // dependent column, below 1e-19, whose tau would overflow
+    if (sig != 0.f && !(av > -FLT_MIN)) {
+      const float tau = -1.f / av;
+      if (live && cl > 0) tw = tau * fmaf(v0, r, dot);
+      r = cl > 0 ? fmaf(-tw, v0, r) : alpha;
+    }
+    float *f = fac + 32 * (j & 1);   // two buffers: one barrier a column
+    f[cl] = -tw;
+    if (live && (W == 32 || !(lane & 1))) R[j * LD + j + cl] = r;
+    __syncwarp();
 #pragma unroll
-    for (int q = 0; q < RPL; ++q) ss = fmaf(x[q], x[q], ss);
-    const float sig = warp_sum_bcast(ss);
-    const float rjj = __shfl_sync(0xffffffffu, r, j);
-    if (sig != 0.f) {   // else the column below the pivot is already zero
-      const float nrm = sqrtf(fmaf(rjj, rjj, sig));
-      const float alpha = rjj > 0.f ? -nrm : nrm;
-      const float v0 = rjj - alpha;
-      const float tau = -1.f / (alpha * v0);
-      float v[32];
+    for (int c4 = 0; c4 < W; c4 += 4) {
+      const float4 t = *reinterpret_cast<const float4 *>(f + c4);
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        float a = 0.f;
+      for (int u = 0; u < 4; ++u) {
+        if (c4 + u == 0) continue;
+        const float tc = u == 0 ? t.x : u == 1 ? t.y : u == 2 ? t.z : t.w;
 #pragma unroll
-        for (int q = 0; q < RPL; ++q) a = fmaf(x[q], p[q][c], a);
-        v[c] = c > j ? a : 0.f;
-      }
-      const float w = fmaf(v0, r, warp_reduce_scatter32(v));
-      const float tw = (lane > j && lane < k) ? tau * w : 0.f;
-      r = fmaf(-tw, v0, r);
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const float twc = __shfl_sync(0xffffffffu, tw, c);
-        if (c > j) {
-#pragma unroll
-          for (int q = 0; q < RPL; ++q) p[q][c] = fmaf(-twc, x[q], p[q][c]);
+        for (int q = 0; q < Q2; ++q) {
+          float2 y = p[q][c4 + u];
+          fma2(y, make_float2(tc, tc), x[q]);
+          p[q][c4 + u - 1] = y;
         }
       }
-      if (lane == j) r = alpha;
     }
-    if (lane < k) R[j * LD + lane] = r;
-    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < Q2; ++q) p[q][W - 1] = make_float2(0.f, 0.f);
   }
+}
+
+template <int LD, int Q2>
+HT_DEV void warp_qr_fold32(float *R, float2 (&p)[Q2][32], int k, float *fac) {
+  if (k > 16) warp_qr_columns<32, LD, Q2>(R, p, 0, 16, k, fac);
+  warp_qr_columns<16, LD, Q2>(R, p, k > 16 ? 16 : 0, k, k, fac);
+  __syncwarp();
 }
 
 // Fold a row-major panel in shared memory (prow <= 64 rows, stride LD) into R.
 template <int KM, int LD>
-HT_DEV void warp_fold_smem(float *R, float *P, int prow, int k) {
+HT_DEV void warp_fold_smem(float *R, float *P, int prow, int k, float *fac) {
   if constexpr (KM == 32) {
     const int lane = threadIdx.x & 31;
-    float p[2][32];
+    float2 p[1][32];
 #pragma unroll
     for (int c = 0; c < 32; ++c) {
-      p[0][c] = (lane < prow && c < k) ? P[lane * LD + c] : 0.f;
-      p[1][c] = (lane + 32 < prow && c < k) ? P[(lane + 32) * LD + c] : 0.f;
+      p[0][c].x = (lane < prow && c < k) ? P[lane * LD + c] : 0.f;
+      p[0][c].y = (lane + 32 < prow && c < k) ? P[(lane + 32) * LD + c] : 0.f;
     }
-    warp_qr_fold32<LD, 2>(R, p, k);
+    warp_qr_fold32<LD, 1>(R, p, k, fac);
   } else {
     warp_qr_fold<KM, LD>(R, P, prow, k);
   }
@@ -214,10 +234,11 @@ __global__ void __launch_bounds__(TqCfg<KM>::THREADS, 1) tsqr_kernel(const TqPar
   constexpr int LD = C::LD;
   extern __shared__ float tq_sm[];
   __shared__ int s_last;
+  __shared__ __align__(16) float facs[C::WARPS][64];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int k = p.k;
   float *R = tq_sm + warp * C::WARP_FLOATS;
-  float *P = R + KM * LD;
+  float *P = R + KM * LD, *fac = facs[warp];
   for (int e = lane; e < KM * LD; e += 32) R[e] = 0.f;
   __syncwarp();
 
@@ -228,15 +249,17 @@ __global__ void __launch_bounds__(TqCfg<KM>::THREADS, 1) tsqr_kernel(const TqPar
        r0 += static_cast<long long>(C::WARPS) * C::PANEL) {
     const int prow = static_cast<int>(min(static_cast<long long>(C::PANEL), r_end - r0));
     if constexpr (KM == 32) {   // the panel straight into registers
-      float pr[TqCfg<KM>::RPL][32];
+      float2 pr[C::RPL / 2][32];
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
         const float *col = p.A + r0 + p.lda * c;
 #pragma unroll
-        for (int q = 0; q < TqCfg<KM>::RPL; ++q)
-          pr[q][c] = (c < k && lane + 32 * q < prow) ? __ldg(col + lane + 32 * q) : 0.f;
+        for (int q = 0; q < C::RPL / 2; ++q) {
+          pr[q][c].x = (c < k && lane + 64 * q < prow) ? __ldg(col + lane + 64 * q) : 0.f;
+          pr[q][c].y = (c < k && lane + 64 * q + 32 < prow) ? __ldg(col + lane + 64 * q + 32) : 0.f;
+        }
       }
-      warp_qr_fold32<LD, TqCfg<KM>::RPL>(R, pr, k);
+      warp_qr_fold32<LD, C::RPL / 2>(R, pr, k, fac);
     } else {
 #pragma unroll 4
       for (int c = 0; c < k; ++c) {
@@ -253,7 +276,7 @@ __global__ void __launch_bounds__(TqCfg<KM>::THREADS, 1) tsqr_kernel(const TqPar
   // 2. the warps' R factors, combined pairwise in shared memory
   auto tree = [&]() {
     for (int half = C::WARPS / 2; half >= 1; half >>= 1) {
-      if (warp < half) warp_fold_smem<KM, LD>(R, tq_sm + (warp + half) * C::WARP_FLOATS, k, k);
+      if (warp < half) warp_fold_smem<KM, LD>(R, tq_sm + (warp + half) * C::WARP_FLOATS, k, k, fac);
       __syncthreads();
     }
   };
@@ -292,7 +315,7 @@ __global__ void __launch_bounds__(TqCfg<KM>::THREADS, 1) tsqr_kernel(const TqPar
     }
     for (int w = warp + C::WARPS; w < gsize; w += C::WARPS) {
       load_member(P, group * TQ_FAN + w);
-      warp_fold_smem<KM, LD>(R, P, k, k);
+      warp_fold_smem<KM, LD>(R, P, k, k, fac);
     }
     __syncthreads();
     tree();
