@@ -883,10 +883,12 @@ ht_status_t leaf_eigs(Ctx &c, const Tree &T, const ht_config_t &cfg, const long 
     // ~10 µs of barriers and pivots, the float-pair factor (~2.5e-4 s^3) and the
     // product (~2e-5 n^2 s), plus the Rayleigh-Ritz Jacobi on s x s.
     int s = std::max(K, std::min<int>({static_cast<int>(n), K + p_over, 64}));
+    bool whole = false;   // the Gram itself: a caller's block (n x (k + oversampling)) plays no part
     if (s < n && n <= 64) {
       const double direct = 2e-3 * n * n * n;
       const double iterate = iters * (10.0 + 2.5e-4 * s * s * s + 2e-5 * n * n * s) + 2e-3 * s * s * s;
-      if (direct <= iterate) s = static_cast<int>(n);
+      whole = direct <= iterate;
+      if (whole) s = static_cast<int>(n);
     }
     if (s > 64) return fail(HT_ERR_UNSUPPORTED, "subspace size above 64");
     EigProblem &e = ep[m];
@@ -900,7 +902,7 @@ ht_status_t leaf_eigs(Ctx &c, const Tree &T, const ht_config_t &cfg, const long 
     e.seed = cfg.seed;
     e.stream_id = static_cast<uint64_t>(m);
     e.start = nullptr;
-    if (cfg.sketch[m]) {
+    if (cfg.sketch[m] && !whole) {
       if (is_device_ptr(cfg.sketch[m])) {
         e.start = cfg.sketch[m];
       } else {
