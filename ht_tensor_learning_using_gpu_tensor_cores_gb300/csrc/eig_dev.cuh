@@ -1332,6 +1332,10 @@ __global__ void __launch_bounds__(256, 1) eig_coop_kernel(const __grid_constant_
   extern __shared__ __align__(16) float sm[];
   const EigSmem m = eig_smem(sm);
 
+  if (static_cast<int>(blockIdx.x) >= B.nsync) {   // past the barrier's members: a direct problem (eig_batched)
+    eig_direct<256>(B.p[B.beside[blockIdx.x - B.nsync]], m);
+    return;
+  }
   int pi = 0;
   while (!(static_cast<int>(blockIdx.x) >= B.p[pi].cta0 && static_cast<int>(blockIdx.x) < B.p[pi].cta0 + B.p[pi].ncta)) ++pi;
   const CoopProb &P = B.p[pi];
@@ -1365,15 +1369,16 @@ __global__ void __launch_bounds__(256, 1) eig_coop_kernel(const __grid_constant_
   eig_iterate<CoopSync, CNS>(P, cl, sy, B.iters, B.refine, m);
 }
 
-// The Jacobi step of every problem, a CTA each: Rayleigh-Ritz of the iterated
-// ones, the whole eigen-decomposition of the direct ones (s == n).  A kernel of
+// The Jacobi step, a CTA per problem: Rayleigh-Ritz of the iterated ones, the
+// whole eigen-decomposition of the direct ones (s == n) that the cooperative
+// kernel did not take.  A kernel of
 // its own so that a round has 32 warps; inside the cooperative kernel, at 8
 // warps, the same step took 172 us on the 48 x 48 matrices of a rank-32
 // decomposition; here 142.
 __global__ void __launch_bounds__(kJacThreads) eig_jacobi_kernel(const __grid_constant__ CoopBatch B) {
   extern __shared__ __align__(16) float sm[];
   const EigSmem m = eig_smem(sm);
-  const CoopProb &P = B.p[blockIdx.x];
+  const CoopProb &P = B.p[B.jacobi[blockIdx.x]];
   if (P.s == P.n) eig_direct<kJacThreads>(P, m);
   else ritz<kJacThreads>(P, m);
 }
