@@ -203,6 +203,7 @@ struct Ctx {
   // FP32 products as three-plane BF16 splits on tcgen05 (tc3_gemm.cu), where
   // the call's workspace holds the planes; off: CUDA cores
   bool tc3 = false;
+  bool planes = false;   // set by a product that takes planes (also in a dry run)
   // X's planes (first mode padded to x3_n1p rows), set by enqueue_body
   const __nv_bfloat16 *x3 = nullptr;
   long long x3_plane = 0;
@@ -1351,6 +1352,7 @@ bool nt_with_planes(const Ctx &c, const NtProduct &p, double min_mac) {
 
 // Operands of a product from planes (arena memory).
 ht_status_t nt_operands(Ctx &c, const NtProduct &p, Gemm3Args *g) {
+  c.planes = true;
   const long long mp = (p.m + 7) / 8 * 8, np = (p.n + 7) / 8 * 8;
   __nv_bfloat16 *a3 = nullptr, *b3 = nullptr;
   HT_TRY(take_planes(c, p.A, p.m, static_cast<long long>(p.k) * p.batch, &a3, &g->a_plane));
@@ -3250,13 +3252,14 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
   for (int m = 0; m < order; ++m) total *= dims[m];
   const bool out_dev = is_device_ptr(x_out);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  bool planes = false;   // a product from planes reads the guard and the error word
   auto plan = [&](Ctx &c) -> ht_status_t {
     const float *Ud[HT_MAX_NODES] = {}, *Bd[HT_MAX_NODES] = {};
     c.err = c.ar.take<int>(64);
     if (!c.err) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small");
     c.nf = c.err + 32;
     c.epoch = 1;
-    if (!c.dry()) HT_CUDA(cudaMemsetAsync(c.err, 0, 64 * sizeof(int), c.st));
+    if (!c.dry() && planes) HT_CUDA(cudaMemsetAsync(c.err, 0, 64 * sizeof(int), c.st));
     HT_TRY(stage_factors(c, T, dims, U, B, Ud, Bd));
     float *o = out_dev ? x_out : c.ar.take<float>(static_cast<size_t>(total));
     if (!o) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small");
@@ -3273,6 +3276,7 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
     d.ar.dry = true;
     d.tc3 = tc3;
     HT_TRY(plan(d));
+    planes = d.planes;
     bytes = d.ar.peak + (1 << 20);
     return acquire_workspace(bytes, &ws, st);
   };
@@ -3290,7 +3294,7 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
   c.ar.cap = bytes;
   HT_TRY(plan(c));
   int errword = 0;
-  HT_CUDA(cudaMemcpyAsync(&errword, c.err, sizeof(int), cudaMemcpyDeviceToHost, c.st));
+  if (planes) HT_CUDA(cudaMemcpyAsync(&errword, c.err, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   HT_CUDA(cudaStreamSynchronize(c.st));
   if (errword & kErrTimeout) return fail(HT_ERR_TIMEOUT, "a kernel's bounded wait expired; results are invalid");
   g_launches += static_cast<unsigned long long>(c.launches);
