@@ -109,11 +109,11 @@ HT_DEV void put_weight(const WeightOut &W, long long e, float v) {
   if (KIND == W_BF16) W.w16[e] = __float2bfloat16_rn(v);
   if (KIND == W_PLANES) {
     const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    const float r = v - __bfloat162float(h);
+    const float r = 128.f * (v - __bfloat162float(h));   // planes as in split_pair
     const __nv_bfloat16 m = __float2bfloat16_rn(r);
     W.w3[e] = h;
     W.w3[W.plane + e] = m;
-    W.w3[2 * W.plane + e] = __float2bfloat16_rn(r - __bfloat162float(m));
+    W.w3[2 * W.plane + e] = __float2bfloat16_rn(128.f * (r - __bfloat162float(m)));
   }
 }
 // An entry without planes (not finite once rounded to BF16): see split3_launch.

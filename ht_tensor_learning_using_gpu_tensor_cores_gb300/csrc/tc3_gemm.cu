@@ -1,7 +1,13 @@
 // FP32-accurate GEMM over tensor matricisations on tcgen05: every FP32 operand
-// is held as three BF16 planes, x = h + m + l exactly (8 significant bits
+// is held as three BF16 planes, x = h + m / 2^7 + l / 2^14 (8 significant bits
 // each), and a product is the six plane products h h', h m', m h', m m', h l',
-// l h' (what is left out, m l' and below, is under 2^-24 of |x x'|).
+// l h' (what is left out, m l' and below, is under 2^-24 of |x x'|).  The lower
+// planes are stored 2^7 and 2^14 times up, because BF16's smallest subnormal is
+// 2^-133 and FP32's last bit 2^-149: the sum is exact for every |x| >= 2^-124 and
+// within 2^-148 of x below that (unscaled planes lose bits from 2^-110 down).  The
+// tensor core takes the factors out again: its accumulator starts with the
+// products 2^14 up and is scaled by 2^-7 as the next group comes in.  |m| and |l|
+// stay below |x| / 2 and |x| / 4, so no sum overflows that h h' does not.
 //
 // What bounds it: the tensor pipe, at six BF16 MMAs per FP32 multiply-add --
 // still several times the CUDA cores' FP32 rate, which the plain FP32 path
@@ -17,8 +23,8 @@
 //
 // Accumulation.  tcgen05 adds into its FP32 accumulator with truncation, so a
 // long K range summed in TMEM would carry a bias of ~2^-24 per step.  The
-// accumulator therefore only ever holds one K block of 64 (small products
-// first, the four h h' steps last); the epilogue warps drain it after every K
+// accumulator therefore only ever holds one K block of 64 (the 2^14 products
+// m m', h l', l h' first, then h m', m h', the four h h' steps last); the epilogue warps drain it after every K
 // block and add it to FP32 sums in registers, rounding to nearest.  Two
 // accumulators take turns, so the drain of one overlaps the MMAs of the other.
 //
@@ -32,7 +38,7 @@
 // warps read the matrix the product is compared with and sum the squared
 // differences (the error pass of a decomposition).
 // Tile 128 x BN; a ring of plane slots (one plane of A and of B, 64 deep in K),
-// filled and freed in the order m, l, h, so that a K block's first slots are
+// filled and freed in the order l, m, h, so that a K block's first slots are
 // refilled while its last products run.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -101,6 +107,16 @@ HT_DEV void tmem_ld_32x32b_x16(uint32_t taddr, float (&v)[16]) {
       : "r"(taddr));
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// D = D / 2^7 + A B^T, as umma_f16 otherwise
+HT_DEV void umma_f16_down7(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.u32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 7;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc)
+      : "memory");
 }
 
 template <int ROWS>
@@ -225,7 +241,7 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
             report_error(p.err, kErrTimeout);
             break;
           }
-          const int kb = kb0 + i / 3, plane = (i % 3 + 1) % 3;   // m, l, h
+          const int kb = kb0 + i / 3, plane = 2 - i % 3;   // l, m, h
           uint8_t *sa = smem + s * C::SLOT;
           mbar_arrive_expect_tx(&full[s], C::SLOT);
           t3_load<T3_BM>(&tmA, p.a_kind, p.a_lblocks, kb, tile.a_row, tile.a_z, plane, sa, &full[s]);
@@ -258,18 +274,19 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
         }
         tc_fence_after();
         const uint32_t d = tmem + static_cast<uint32_t>(set * BN);
-        const int sm = it % NSLOT, sl = (it + 1) % NSLOT, sh = (it + 2) % NSLOT;
+        const int sl = it % NSLOT, sm = (it + 1) % NSLOT, sh = (it + 2) % NSLOT;
         const uint32_t am = smem_u32(smem + sm * C::SLOT), al = smem_u32(smem + sl * C::SLOT),
                        ah = smem_u32(smem + sh * C::SLOT);
         // 16-wide K steps that hold data (the rest of the block is zero fill)
         const int kb = kb0 + i;
         const long long left = p.a_len - static_cast<long long>(p.a_kind == OP_MN3 ? kb : kb % p.a_lblocks) * T3_BK;
         const int steps = left >= T3_BK ? T3_BK / 16 : max(1, (static_cast<int>(left) + 15) / 16);
-        bool first = true;
-        auto product = [&](uint32_t a, uint32_t b) {
+        // D = (down ? D / 2^7 : D or nothing) + a b over the block's steps
+        auto product = [&](uint32_t a, uint32_t b, bool fresh, bool down) {
           for (int kk = 0; kk < steps; ++kk) {
-            umma_f16(d, t3_desc(p.a_kind, a, kk), t3_desc(p.b_kind, b + C::A_BYTES, kk), idesc, first ? 0u : 1u);
-            first = false;
+            const uint64_t da = t3_desc(p.a_kind, a, kk), db = t3_desc(p.b_kind, b + C::A_BYTES, kk);
+            if (down && kk == 0) umma_f16_down7(d, da, db, idesc);
+            else umma_f16(d, da, db, idesc, fresh && kk == 0 ? 0u : 1u);
           }
         };
         auto ready = [&](int j) {
@@ -278,18 +295,18 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
           report_error(p.err, kErrTimeout);
           return false;
         };
-        if (!ready(it)) break;
+        if (!ready(it) || !ready(it + 1)) break;
         tc_fence_after();
-        product(am, am);
-        if (!ready(it + 1) || !ready(it + 2)) break;
+        product(am, am, true, false);
+        if (!ready(it + 2)) break;
         tc_fence_after();
-        product(ah, am);
-        product(am, ah);
-        umma_commit(&empty[sm]);
-        product(ah, al);
-        product(al, ah);
+        product(ah, al, false, false);
+        product(al, ah, false, false);
         umma_commit(&empty[sl]);
-        product(ah, ah);
+        product(ah, am, false, true);
+        product(am, ah, false, false);
+        umma_commit(&empty[sm]);
+        product(ah, ah, false, true);
         umma_commit(&empty[sh]);
         umma_commit(&tfull[set]);
         ok = true;
@@ -433,12 +450,13 @@ HT_DEV uint32_t pack2(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&v);
 }
-// (h, m, l) of a pair; each rest x - h, x - h - m is exact
+// (h, m, l) of a pair; each rest is exact, and so are the factors (a rest is at
+// most half a unit of its plane's last place)
 HT_DEV void split_pair(float x, float y, uint32_t &h, uint32_t &m, uint32_t &l) {
   h = pack2(x, y);
-  const float rx = x - __uint_as_float(h << 16), ry = y - __uint_as_float(h & 0xffff0000u);
+  const float rx = 128.f * (x - __uint_as_float(h << 16)), ry = 128.f * (y - __uint_as_float(h & 0xffff0000u));
   m = pack2(rx, ry);
-  l = pack2(rx - __uint_as_float(m << 16), ry - __uint_as_float(m & 0xffff0000u));
+  l = pack2(128.f * (rx - __uint_as_float(m << 16)), 128.f * (ry - __uint_as_float(m & 0xffff0000u)));
 }
 
 // Block sum of the compensated sums of squares -> partials[blockIdx.x].
