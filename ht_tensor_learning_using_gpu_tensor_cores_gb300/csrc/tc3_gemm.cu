@@ -138,45 +138,190 @@ HT_DEV uint64_t t3_desc(int kind, uint32_t base, int kk) {
 }
 
 // The launch's product from its FP32 operands, when an entry had no planes
-// (split3_kernel): a thread forms 4 rows of one column of a tile at a time,
-// straight from global memory.  Not tuned: it runs on data with infinities or
-// NaN, where only the FP32 result's own infinities and NaN matter.
-template <int BN>
-__device__ __noinline__ void t3_fallback(const T3Params &p, const TileGen &gen) {
-  for (int w = blockIdx.x; w < p.work; w += gridDim.x) {
-    const int tile_idx = w % p.num_tiles, split = w / p.num_tiles;
-    const Tile tile = gen_tile(gen, tile_idx);
-    const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
-    for (int e = threadIdx.x; e < T3_BM / 4 * BN; e += blockDim.x) {
-      const int row0 = (e % (T3_BM / 4)) * 4, col = e / (T3_BM / 4);
-      const bool live_col = col < tile.valid_cols;
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int kb = kb0; kb < kb1 && live_col; ++kb) {
-        const bool amn = p.a_kind == OP_MN3, bmn = p.b_kind == OP_MN3;
-        const long long al = static_cast<long long>(amn ? kb : kb % p.a_lblocks) * T3_BK, ar = amn ? 0 : kb / p.a_lblocks;
-        const long long bl = static_cast<long long>(bmn ? kb : kb % p.b_lblocks) * T3_BK, br = bmn ? 0 : kb / p.b_lblocks;
-        const long long n = min(static_cast<long long>(T3_BK), min(p.a32.len - al, p.b32.len - bl));
-        const float *a = p.a32.p + al * p.a32.ls + ar * p.a32.rr + tile.a_z * p.a32.zs + (tile.a_row + row0) * p.a32.rs;
-        const float *b = p.b32.p + bl * p.b32.ls + br * p.b32.rr + static_cast<long long>(tile.b_row + col) * p.b32.rs;
-        for (long long l = 0; l < n; ++l) {
-          const float y = __ldg(b + l * p.b32.ls);
+// (split3_kernel).  Data with infinities or NaN comes in earnest (a diverged
+// training step), so its call has to stay near the CUDA cores' rate: for the
+// forward of 8192 x 1024 x 1024 a thread per four outputs straight from global
+// memory took 36.9 ms, this takes 0.97 and simt_gemm_kernel's tiles 0.67.
+// Parts of SC columns of a tile are walked with 32-deep slices of both operands
+// in two shared-memory stages, the next slice (also the next part's first) on its
+// way in registers; a thread forms 8 rows x 4 columns.
+template <int BN, int NSLOT>
+struct T3Fallback {
+  using C = T3Cfg<BN, NSLOT>;
+  static constexpr int NT = 32 * C::EW, SC = NT / 4, SUB = BN / SC, KC = T3_BK / 2;
+  static constexpr int LDA = T3_BM + 4, LDB = SC + 4, STAGE = KC * (LDA + LDB);   // floats
+  static_assert(2 * STAGE * sizeof(float) <= size_t(NSLOT) * C::SLOT, "two stages in the ring's memory");
+};
+
+// A thread's quads of the ROWS x KC slice of one operand: four consecutive
+// entries along whichever index is contiguous, neighbouring threads on
+// neighbouring quads.  Entry (i, l) is kept at row l, with the groups of four i
+// permuted by l's group, so that storing quads along l meets no bank twice.
+HT_DEV int t3_group(int g, int l) { return 4 * (g ^ ((l >> 2) & 7)); }
+template <int ROWS, int LD, int THREADS>
+struct T3Slice {
+  static constexpr int KC = T3_BK / 2, QUADS = ROWS * KC / 4, NV = (QUADS + THREADS - 1) / THREADS;
+  float4 v[NV];
+  // entries i < n_rows, l < n_l of src (steps rs, ls); zeros past them
+  HT_DEV void load(const float *src, long long rs, long long ls, int n_rows, int n_l) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (row0 + i < tile.valid_rows) s[i] = fmaf(__ldg(a + l * p.a32.ls + i * p.a32.rs), y, s[i]);
-        }
+    for (int q = 0; q < NV; ++q) {
+      const int e = threadIdx.x + q * THREADS;
+      const int i = rs == 1 ? 4 * (e % (ROWS / 4)) : e / (KC / 4), l = rs == 1 ? e / (ROWS / 4) : 4 * (e % (KC / 4));
+      v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (e >= QUADS || i >= n_rows || l >= n_l) continue;
+      const float *from = src + i * rs + l * ls;
+      const int n = rs == 1 ? n_rows - i : n_l - l;   // entries of the quad inside the slice
+      if (n >= 4 && (reinterpret_cast<uintptr_t>(from) & 15u) == 0) {
+        v[q] = __ldg(reinterpret_cast<const float4 *>(from));
+      } else {
+        v[q].x = __ldg(from);
+        if (n > 1) v[q].y = __ldg(from + 1);
+        if (n > 2) v[q].z = __ldg(from + 2);
+        if (n > 3) v[q].w = __ldg(from + 3);
       }
+    }
+  }
+  HT_DEV void store(bool rows_contiguous, float *dst) const {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int row = row0 + i;
-        if (p.out_mode == OUT_PARTIAL) {
-          p.out[((static_cast<size_t>(split) * p.num_tiles + tile_idx) * T3_BM + row) * BN + col] = s[i];
-        } else if (row < tile.valid_rows && live_col) {
-          float v = p.bias ? s[i] + p.bias[tile.out_row + row] : s[i];
-          if (p.relu) v = fmaxf(v, 0.f);
-          p.out[tile.out_row + row + p.ld_out * static_cast<long long>(tile.out_col + col)] = v;
+    for (int q = 0; q < NV; ++q) {
+      const int e = threadIdx.x + q * THREADS;
+      if (e >= QUADS) continue;
+      if (rows_contiguous) {
+        const int l = e / (ROWS / 4);
+        *reinterpret_cast<float4 *>(dst + l * LD + t3_group(e % (ROWS / 4), l)) = v[q];
+      } else {
+        const int i = e / (KC / 4), l = 4 * (e % (KC / 4));
+        float *d = dst + l * LD + t3_group(i >> 2, l) + (i & 3);
+        d[0] = v[q].x;
+        d[LD] = v[q].y;
+        d[2 * LD] = v[q].z;
+        d[3 * LD] = v[q].w;
+      }
+    }
+  }
+};
+
+template <int BN, int NSLOT>
+__device__ __noinline__ void t3_fallback(const T3Params &p, const TileGen &gen, float *sm) {
+  using F = T3Fallback<BN, NSLOT>;
+  constexpr int THREADS = F::C::THREADS;
+  const int t = threadIdx.x, rg = t % 16, cg = t / 16;
+  const long long ars = p.a32.rs, als = p.a32.ls, brs = p.b32.rs, bls = p.b32.ls;
+  // part w: columns [col0, col0 + SC) of item w / SUB's tile
+  auto part = [&](int w, int &col0, int &tile_idx, int &split) {
+    const int item = w / F::SUB;
+    col0 = w % F::SUB * F::SC;
+    tile_idx = item % p.num_tiles;
+    split = item / p.num_tiles;
+    return gen_tile(gen, tile_idx);
+  };
+  // the slice being fetched: slice i of part w, n deep
+  int w = blockIdx.x, i = 0, n = 0, slices = 0, kb0 = 0, rows = 0, cols = 0;
+  const float *arow = nullptr, *brow = nullptr;
+  const float *a = nullptr, *b = nullptr;
+  const int parts = p.work * F::SUB;
+  auto locate = [&]() {   // slice i's entries and depth
+    const bool amn = p.a_kind == OP_MN3, bmn = p.b_kind == OP_MN3;
+    const int kb = kb0 + i / 2, h = (i & 1) * F::KC;
+    const int ar = amn ? 0 : kb / p.a_lblocks, br = bmn ? 0 : kb / p.b_lblocks;
+    const long long al = (kb - static_cast<long long>(ar) * p.a_lblocks * !amn) * T3_BK + h;
+    const long long bl = (kb - static_cast<long long>(br) * p.b_lblocks * !bmn) * T3_BK + h;
+    n = static_cast<int>(max(0ll, min(static_cast<long long>(F::KC), min(p.a32.len - al, p.b32.len - bl))));
+    a = arow + al * als + ar * p.a32.rr;
+    b = brow + bl * bls + br * p.b32.rr;
+  };
+  auto open = [&]() {   // part w, or the next of this CTA's that has columns
+    for (; w < parts; w += gridDim.x) {
+      int col0, tile_idx, split;
+      const Tile tile = part(w, col0, tile_idx, split);
+      if (p.out_mode != OUT_PARTIAL && col0 >= tile.valid_cols) continue;
+      rows = tile.valid_rows;
+      cols = tile.valid_cols - col0;
+      arow = p.a32.p + tile.a_z * p.a32.zs + tile.a_row * ars;
+      brow = p.b32.p + (tile.b_row + col0) * brs;
+      kb0 = split * p.kb_per_split;
+      slices = 2 * max(0, min(p.num_kb, kb0 + p.kb_per_split) - kb0);
+      i = n = 0;
+      if (slices) locate();   // (a split without K blocks: zeros)
+      return;
+    }
+  };
+  auto advance = [&]() {
+    while (++i < slices) {
+      locate();
+      if (n > 0) return;
+    }
+    w += gridDim.x;
+    open();
+  };
+  T3Slice<T3_BM, F::LDA, THREADS> sa;
+  T3Slice<F::SC, F::LDB, THREADS> sb;
+  float2 acc[4][4];   // [column][pair of rows: 4 rg, 4 rg + 2, 64 + 4 rg, ...]
+  auto clear = [&]() {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[j][r] = make_float2(0.f, 0.f);
+  };
+  clear();
+  open();
+  if (w < parts) {
+    sa.load(a, ars, als, rows, n);
+    sb.load(b, brs, bls, cols, n);
+  }
+  for (int stage = 0; w < parts; stage ^= 1) {
+    float *As = sm + stage * F::STAGE, *Bs = As + F::KC * F::LDA;
+    sa.store(ars == 1, As);
+    sb.store(brs == 1, Bs);
+    __syncthreads();   // (and the other stage's slice is used up)
+    const int w0 = w, n0 = n;
+    advance();
+    if (w < parts) {
+      sa.load(a, ars, als, rows, n);
+      sb.load(b, brs, bls, cols, n);
+    }
+    if (t >= F::NT) continue;
+#pragma unroll 4
+    for (int l = 0; l < n0; ++l) {
+      const float4 a0 = *reinterpret_cast<const float4 *>(As + l * F::LDA + t3_group(rg, l));
+      const float4 a1 = *reinterpret_cast<const float4 *>(As + l * F::LDA + 64 + t3_group(rg, l));
+      const float4 b4 = *reinterpret_cast<const float4 *>(Bs + l * F::LDB + t3_group(cg, l));
+      const float bj[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 x = make_float2(bj[j], bj[j]);
+        fma2(acc[j][0], x, make_float2(a0.x, a0.y));
+        fma2(acc[j][1], x, make_float2(a0.z, a0.w));
+        fma2(acc[j][2], x, make_float2(a1.x, a1.y));
+        fma2(acc[j][3], x, make_float2(a1.z, a1.w));
+      }
+    }
+    if (w == w0) continue;
+    int col0, tile_idx, split;   // that was the part's last slice
+    const Tile tile = part(w0, col0, tile_idx, split);
+    const int col = col0 + 4 * cg;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int row = (r < 4 ? 0 : 64) + 4 * rg + (r & 3);
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = r & 1 ? acc[j][r / 2].y : acc[j][r / 2].x;
+      if (p.out_mode == OUT_PARTIAL) {
+        float *dst = p.out + ((static_cast<size_t>(split) * p.num_tiles + tile_idx) * T3_BM + row) * BN + col;
+        *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+      } else if (row < tile.valid_rows) {
+        const float bias = p.bias ? p.bias[tile.out_row + row] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (p.bias) v[j] += bias;
+          if (p.relu) v[j] = fmaxf(v[j], 0.f);
+          if (col + j < tile.valid_cols)
+            p.out[tile.out_row + row + p.ld_out * static_cast<long long>(tile.out_col + col + j)] = v[j];
         }
       }
     }
+    clear();
   }
 }
 
@@ -197,7 +342,7 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   if (p.guard && *p.guard == p.epoch) {   // the same answer in every thread of the grid
-    t3_fallback<BN>(p, gen);
+    t3_fallback<BN, NSLOT>(p, gen, reinterpret_cast<float *>(smem));
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -616,11 +761,14 @@ cudaError_t t3_launch(const Gemm3Args &g, cudaStream_t s) {
   p.a_len = g.a.kind == OP_MN3 ? g.a.d1 : g.a.d0;
   p.a32 = g.a32;
   p.b32 = g.b32;
-  p.guard = g.guard;
+  p.guard = g.out_mode == OUT_SQDIFF ? nullptr : g.guard;   // (the fallback stores its product)
   p.epoch = g.epoch;
   p.bias = g.bias;
   p.relu = g.relu;
-  tc3_gemm_kernel<BN, NSLOT, MINB><<<tc3_grid(p.work), C::THREADS, C::SMEM, s>>>(ma, mb, p, g.gen);
+  // guarded: enough CTAs for the fallback's parts of the tiles
+  const int grid = p.guard ? int(std::min<long long>((long long)p.work * T3Fallback<BN, NSLOT>::SUB, device_sm_count()))
+                           : tc3_grid(p.work);
+  tc3_gemm_kernel<BN, NSLOT, MINB><<<grid, C::THREADS, C::SMEM, s>>>(ma, mb, p, g.gen);
   return cudaGetLastError();
 }
 
