@@ -208,10 +208,10 @@ struct Ctx {
   const __nv_bfloat16 *x3 = nullptr;
   long long x3_plane = 0;
   long x3_n1p = 0;
-  // entries without planes (not finite): *nf == epoch makes the guarded FP32
-  // kernel form the product again (null: the caller rejects such data itself)
+  // entries without planes (not finite) set *nf, which makes the products take
+  // their FP32 operands (null: the caller rejects such data itself).  The call's
+  // first work on the stream clears it, so that a recorded call can be replayed.
   int *nf = nullptr;
-  int epoch = 0;
   int eig_ctas = 0;     // cap on the cooperative eigen-solver's grid (0 = every SM)
   // Staged enqueue of the batched path.  eig_mode 0: leaf_eigs launches the
   // cooperative solver; 1: it appends its problems to eig_table (the grouped
@@ -508,7 +508,6 @@ ht_status_t run_gemm3(Ctx &c, const GemmReq &q) {
   g.a32 = fp32_operand(q.a32);
   g.b32 = fp32_operand(q.b32);
   g.guard = c.nf;
-  g.epoch = c.epoch;
   g.bias = partial ? nullptr : q.bias;
   g.relu = !partial && q.relu ? 1 : 0;
   HT_CUDA(tc3_gemm_launch(g, c.st));
@@ -548,7 +547,7 @@ ht_status_t take_planes(Ctx &c, const float *x, long long rows, long long cols, 
   *out = c.ar.take<__nv_bfloat16>(static_cast<size_t>(3 * *plane));
   if (!*out) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small (operand planes)");
   if (c.dry()) return HT_OK;
-  HT_CUDA(split3_launch(x, *out, *plane, rows, rp, cols, partials, num_partials, c.nf, c.epoch, c.st));
+  HT_CUDA(split3_launch(x, *out, *plane, rows, rp, cols, partials, num_partials, c.nf, c.st));
   ++c.launches;
   return HT_OK;
 }
@@ -1381,7 +1380,6 @@ ht_status_t nt_operands(Ctx &c, const NtProduct &p, Gemm3Args *g) {
   g->b32.p = p.B;
   g->b32.rs = 1; g->b32.ls = p.n; g->b32.len = p.k;
   g->guard = c.nf;
-  g->epoch = c.epoch;
   return HT_OK;
 }
 
@@ -3258,7 +3256,6 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
     c.err = c.ar.take<int>(64);
     if (!c.err) return fail(HT_ERR_OUT_OF_MEMORY, "workspace too small");
     c.nf = c.err + 32;
-    c.epoch = 1;
     if (!c.dry() && planes) HT_CUDA(cudaMemsetAsync(c.err, 0, 64 * sizeof(int), c.st));
     HT_TRY(stage_factors(c, T, dims, U, B, Ud, Bd));
     float *o = out_dev ? x_out : c.ar.take<float>(static_cast<size_t>(total));
@@ -3801,7 +3798,6 @@ namespace {
 
 std::mutex g_layer_mutex;
 DeviceWorkspace g_layer_ws[64];
-int g_layer_epoch[64];  // calls since the workspace was made (Ctx::epoch)
 int *g_layer_err[64];   // first 256 bytes of each device's layer workspace
 
 ht_status_t layer_shape(const ht_layer_shape_t *in, LayerShape *sh) {
@@ -3883,7 +3879,6 @@ ht_status_t layer_run(cudaStream_t st, bool tc, F &&plan) {
     HT_CUDA(cudaDeviceSynchronize());
     w.bytes = bytes;
     g_layer_err[dev] = static_cast<int *>(w.ptr);
-    g_layer_epoch[dev] = 0;
   }
   Ctx c;
   c.st = st;
@@ -3891,7 +3886,6 @@ ht_status_t layer_run(cudaStream_t st, bool tc, F &&plan) {
   c.tc3 = tc3;
   c.err = g_layer_err[dev];
   c.nf = g_layer_err[dev] + 32;   // its own 128 bytes behind the error word
-  c.epoch = ++g_layer_epoch[dev];
   c.ar.base = static_cast<char *>(w.ptr) + 256;
   c.ar.cap = w.bytes - 256;
   HT_TRY(plan(c));
@@ -3974,8 +3968,8 @@ ht_status_t ht_layer_weight(const ht_layer_shape_t *shape, const float *u1, cons
     float *Q = c.ar.take<float>(layer_q_count(sh));
     if (!P || !Q) return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
     if (c.dry()) return HT_OK;
-    HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st));
-    HT_CUDA(layer_weight_launch(sh, P, Q, W, nullptr, nullptr, 0, nullptr, 0, c.st));
+    HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st, nullptr));
+    HT_CUDA(layer_weight_launch(sh, P, Q, W, nullptr, nullptr, 0, nullptr, c.st));
     c.launches += 2;
     return HT_OK;
   });
@@ -4007,8 +4001,8 @@ ht_status_t ht_layer_forward(const ht_layer_shape_t *shape, const float *u1, con
     if (c.tc3 && nin % 8 == 0) HT_TRY(reserve_planes(c, nin, nout, &W3));
     if (!P || !Q || !(W32 || W16) || (tc && !x16)) return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
     if (!c.dry()) {
-      HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st));
-      HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.epoch, c.st));
+      HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st, c.nf));
+      HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.st));
       if (tc) HT_CUDA(f32_to_bf16_launch(x, x16, batch * nin, c.st));
       c.launches += tc ? 3 : 2;
     }
@@ -4063,10 +4057,10 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
       HT_TRY(reserve_planes(c, nout, batch, &dy3));
     }
     if (!c.dry()) {
-      HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, T1, c.st, dbias ? dy : nullptr, batch, part));
+      HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, T1, c.st, c.nf, dbias ? dy : nullptr, batch, part));
       ++c.launches;
       if (dx) {
-        HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.epoch, c.st));
+        HT_CUDA(layer_weight_launch(sh, P, Q, W32, W16, W3.p, W3.plane, c.nf, c.st));
         ++c.launches;
       }
       if (tc) {
@@ -4077,12 +4071,11 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
     }
     if (x3.p && !c.dry()) {
       if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 15u) == 0) {
-        HT_CUDA(split3_pair_launch(x, x3.p, x3.plane, batch * nin, dy, dy3.p, dy3.plane, batch * nout, c.nf, c.epoch,
-                                   c.st));
+        HT_CUDA(split3_pair_launch(x, x3.p, x3.plane, batch * nin, dy, dy3.p, dy3.plane, batch * nout, c.nf, c.st));
         ++c.launches;
       } else {
-        HT_CUDA(split3_launch(x, x3.p, x3.plane, nin, nin, batch, nullptr, 0, c.nf, c.epoch, c.st));
-        HT_CUDA(split3_launch(dy, dy3.p, dy3.plane, nout, nout, batch, nullptr, 0, c.nf, c.epoch, c.st));
+        HT_CUDA(split3_launch(x, x3.p, x3.plane, nin, nin, batch, nullptr, 0, c.nf, c.st));
+        HT_CUDA(split3_launch(dy, dy3.p, dy3.plane, nout, nout, batch, nullptr, 0, c.nf, c.st));
         c.launches += 2;
       }
     }

@@ -119,11 +119,10 @@ struct Fp32Operand {
 };
 struct Gemm3Args {
   Operand a, b;
-  // non-null guard: *guard == epoch (an operand entry had no planes, see
+  // non-null guard: *guard != 0 (an operand entry had no planes, see
   // split3_launch) makes the launch form the product from a32, b32 instead
   Fp32Operand a32, b32;
   const int *guard = nullptr;
-  int epoch = 0;
   long long a_plane, b_plane;
   TileGen gen;
   int splits, out_mode;
@@ -141,14 +140,14 @@ cudaError_t tc3_gemm_launch(const Gemm3Args &g, cudaStream_t s);
 long tc3_num_kblocks(const Operand &a);
 // x (n1 x rest) -> three planes of n1p x rest (zero rows n1 <= i < n1p), n1p a
 // multiple of 8; partials non-null: also num_partials block sums of squares;
-// flag non-null: *flag = epoch when an entry has no planes (not finite).
+// flag non-null: *flag = 1 when an entry has no planes (not finite).
 // A second array (x2, elements in multiples of 8, 16-byte aligned like x) can
 // ride along when x needs no padding and no sums.
 cudaError_t split3_pair_launch(const float *x, __nv_bfloat16 *planes, long long plane, long long n, const float *x2,
-                               __nv_bfloat16 *planes2, long long plane2, long long n2, int *flag, int epoch,
+                               __nv_bfloat16 *planes2, long long plane2, long long n2, int *flag,
                                cudaStream_t s);
 cudaError_t split3_launch(const float *x, __nv_bfloat16 *planes, long long plane, long long n1, long long n1p,
-                          long long rest, double *partials, int num_partials, int *flag, int epoch, cudaStream_t s);
+                          long long rest, double *partials, int num_partials, int *flag, cudaStream_t s);
 
 // SIMT FP32 path (float operands), BM = 128, BN in {64, 128}.
 // Grouped FP32 GEMMs of the batched path (the 3rd-order core pass): every
@@ -472,13 +471,14 @@ struct LayerShape {
   int r1, r2, r3, r4;
 };
 // P[a, b, r1] (A x B x r1), Q[c, r1] (C x r1) and, when T1 is non-null,
-// T1[a, r4, r1] = sum_r3 u1[a, r3] b2[r3, r4, r1]
+// T1[a, r4, r1] = sum_r3 u1[a, r3] b2[r3, r4, r1].  clear (or null): a word set to
+// zero -- the call's guard, before the launches that may set it
 cudaError_t layer_pq_launch(const LayerShape &sh, const float *u1, const float *u2, const float *u3, const float *b2,
-                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s, const float *dy = nullptr,
-                            long long batch = 0, float *cpart = nullptr);
+                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s, int *clear,
+                            const float *dy = nullptr, long long batch = 0, float *cpart = nullptr);
 // W (Nout x Nin, row-major) from P and Q, into W32 (FP32) or, when W32 is null, W16 (BF16)
 cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
-                                __nv_bfloat16 *W3, long long plane, int *flag, int epoch, cudaStream_t s);
+                                __nv_bfloat16 *W3, long long plane, int *flag, cudaStream_t s);
 // y[z, o] = act(y[z, o] + bias[o]) (bias may be null; act 0 identity, 1 ReLU)
 cudaError_t bias_act_launch(float *y, const float *bias, long long batch, long long nout, int act, cudaStream_t s);
 // Ranges of the batch whose partial column sums of dy layer_factor_grads_launch

@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(kLayerThreads) layer_pq_kernel(const LayerShap
                                                                  const float *__restrict__ b2,
                                                                  const float *__restrict__ b1, float *__restrict__ P,
                                                                  float *__restrict__ Q, float *__restrict__ T1g,
-                                                                 int npq, const ColsumArgs cs) {
+                                                                 int npq, const ColsumArgs cs, int *clear) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && clear) *clear = 0;
   if (static_cast<int>(blockIdx.x) >= npq) {
     layer_colsum_body(cs.dy, cs.batch, cs.nout, cs.chunks, cs.part, blockIdx.x - npq);
     return;
@@ -124,7 +125,7 @@ HT_DEV bool no_planes(float v) { return !(fabsf(__bfloat162float(__float2bfloat1
 template <int KIND>
 __global__ void __launch_bounds__(kLayerThreads) layer_weight_kernel(const LayerShape sh, const float *__restrict__ P,
                                                                      const float *__restrict__ Q, const WeightOut W,
-                                                                     int *flag, int epoch) {
+                                                                     int *flag) {
   const int N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
   const long long Nin = static_cast<long long>(sh.n[0]) * N1 * N2, Nout = static_cast<long long>(M0) * M1 * M2;
   const int B = N1 * M1, R1 = sh.r1;
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(kLayerThreads) layer_weight_kernel(const Layer
     float s = 0.f;
     for (int r = 0; r < R1; ++r) s = fmaf(p[r], q[r], s);
     put_weight<KIND>(W, e, s);
-    if (KIND == W_PLANES && no_planes(s)) *flag = epoch;
+    if (KIND == W_PLANES && no_planes(s)) *flag = 1;
   }
 }
 
@@ -153,7 +154,7 @@ template <int KIND, int RB>
 __global__ void __launch_bounds__(kLayerThreads, RB < 64 ? 3 : 1) layer_weight_tiled_kernel(const LayerShape sh,
                                                                            const float *__restrict__ P,
                                                                            const float *__restrict__ Q,
-                                                                           const WeightOut W, int *flag, int epoch) {
+                                                                           const WeightOut W, int *flag) {
   constexpr int G = 64 / RB;
   extern __shared__ __align__(16) float Ps[];   // NP x RB, zero past R1; behind it Qs: N2 rows of 65
   const int N0 = sh.n[0], N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(kLayerThreads, RB < 64 ? 3 : 1) layer_weight_t
         }
     }
   }
-  if (KIND == W_PLANES && bad) *flag = epoch;
+  if (KIND == W_PLANES && bad) *flag = 1;
 }
 
 // y[z, o] = act(y[z, o] + bias[o]), act 0 = identity, 1 = ReLU
@@ -638,14 +639,14 @@ __global__ void __launch_bounds__(kLayerThreads) layer_grads_kernel(const LayerS
 }  // namespace
 
 cudaError_t layer_pq_launch(const LayerShape &sh, const float *u1, const float *u2, const float *u3, const float *b2,
-                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s, const float *dy,
-                            long long batch, float *cpart) {
+                            const float *b1, float *P, float *Q, float *T1, cudaStream_t s, int *clear,
+                            const float *dy, long long batch, float *cpart) {
   const int A = sh.n[0] * sh.m[0], C = sh.n[2] * sh.m[2];
   const long long qb = (static_cast<long long>(C) * sh.r1 + kLayerThreads - 1) / kLayerThreads;
   const ColsumArgs cs{dy, batch, static_cast<long long>(sh.m[0]) * sh.m[1] * sh.m[2], layer_colsum_chunks(batch), cpart};
   const long long ncol = dy ? (cs.nout + kLayerThreads - 1) / kLayerThreads * cs.chunks : 0;
   layer_pq_kernel<<<static_cast<unsigned>(A + qb + ncol), kLayerThreads, 0, s>>>(sh, u1, u2, u3, b2, b1, P, Q, T1,
-                                                                                static_cast<int>(A + qb), cs);
+                                                                                static_cast<int>(A + qb), cs, clear);
   return cudaGetLastError();
 }
 
@@ -671,7 +672,7 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 }
 
 template <int KIND>
-cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, const WeightOut &W, int *flag, int epoch,
+cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, const WeightOut &W, int *flag,
                           cudaStream_t s) {
   const long long total = static_cast<long long>(sh.n[0]) * sh.n[1] * sh.n[2] * sh.m[0] * sh.m[1] * sh.m[2];
   const size_t smem = layer_weight_smem(sh);
@@ -680,7 +681,7 @@ cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, 
     const unsigned grid = static_cast<unsigned>(sh.m[0]) * sh.m[1] * ((sh.m[2] + G - 1) / G);
     auto launch = [&](auto kernel) -> cudaError_t {
       const cudaError_t e = allow_smem(kernel, smem);
-      if (e == cudaSuccess) kernel<<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W, flag, epoch);
+      if (e == cudaSuccess) kernel<<<grid, kLayerThreads, smem, s>>>(sh, P, Q, W, flag);
       return e;
     };
     const cudaError_t e = rb == 16   ? launch(layer_weight_tiled_kernel<KIND, 16>)
@@ -688,17 +689,17 @@ cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, 
                                      : launch(layer_weight_tiled_kernel<KIND, 64>);
     if (e != cudaSuccess) return e;
   } else {
-    layer_weight_kernel<KIND><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W, flag, epoch);
+    layer_weight_kernel<KIND><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W, flag);
   }
   return cudaGetLastError();
 }
 
 cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
-                                __nv_bfloat16 *W3, long long plane, int *flag, int epoch, cudaStream_t s) {
+                                __nv_bfloat16 *W3, long long plane, int *flag, cudaStream_t s) {
   const WeightOut W{W32, W16, W3, plane};
-  if (W3) return W32 && flag ? weight_launch<W_PLANES>(sh, P, Q, W, flag, epoch, s) : cudaErrorInvalidValue;
-  if (W32) return weight_launch<W_FP32>(sh, P, Q, W, flag, epoch, s);
-  return weight_launch<W_BF16>(sh, P, Q, W, flag, epoch, s);
+  if (W3) return W32 && flag ? weight_launch<W_PLANES>(sh, P, Q, W, flag, s) : cudaErrorInvalidValue;
+  if (W32) return weight_launch<W_FP32>(sh, P, Q, W, flag, s);
+  return weight_launch<W_BF16>(sh, P, Q, W, flag, s);
 }
 
 cudaError_t bias_act_launch(float *y, const float *bias, long long batch, long long nout, int act, cudaStream_t s) {

@@ -77,9 +77,8 @@ struct T3Params {
   int *err;
   double *parts;                // OUT_SQDIFF: one sum of squared differences per CTA
   long long a_len;              // extent of A's contiguous K run: d0 (K-major) or d1 (MN-major)
-  Fp32Operand a32, b32;         // read when *guard == epoch (see t3_fallback)
+  Fp32Operand a32, b32;         // read when *guard is set (see t3_fallback)
   const int *guard;
-  int epoch;
   const float *bias;            // added to row r of a column-major output (bias[out_row + r]), or null
   int relu;
 };
@@ -341,7 +340,7 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-  if (p.guard && *p.guard == p.epoch) {   // the same answer in every thread of the grid
+  if (p.guard && *p.guard != 0) {   // the same answer in every thread of the grid
     t3_fallback<BN, NSLOT>(p, gen, reinterpret_cast<float *>(smem));
     return;
   }
@@ -621,15 +620,15 @@ HT_DEV void block_sumsq(const Acc2 &a, double *partials) {
 // An entry whose first plane is not finite (NaN, infinite, or rounded up past
 // the largest BF16) has no three-plane form: infinity minus infinity in its
 // lower planes would turn every product it meets into NaN.  Such an entry
-// stores `epoch` in *flag, and the product's launch then takes its FP32
-// operands instead (t3_fallback).
+// sets *flag, which the caller's first launch cleared, and the product's launch
+// then takes its FP32 operands instead (t3_fallback).
 // A thread forms 8 consecutive elements of all planes: one 16-byte store per
 // plane, and two 16-byte loads when x's rows are 16-byte aligned (VEC).  Bound
 // by HBM: 4 B read and 6 B written per element.
 template <bool VEC, bool SQ>
 __global__ void __launch_bounds__(256) split3_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ planes,
                                                      long long plane, long long n1, long long n1p, long long rest,
-                                                     double *partials, int *flag, int epoch) {
+                                                     double *partials, int *flag) {
   Acc2 a = {0.f, 0.f};
   bool bad = false;
   const long long v1 = n1p / 8, total = v1 * rest;
@@ -659,7 +658,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const float *__restrict__ x
     *reinterpret_cast<uint4 *>(planes + plane + 8 * e) = make_uint4(m[0], m[1], m[2], m[3]);
     *reinterpret_cast<uint4 *>(planes + 2 * plane + 8 * e) = make_uint4(l[0], l[1], l[2], l[3]);
   }
-  if (flag && bad) *flag = epoch;   // every writer stores the same value
+  if (flag && bad) *flag = 1;   // every writer stores the same value
   if (SQ) block_sumsq(a, partials);
 }
 
@@ -669,7 +668,7 @@ struct SplitJob {
   __nv_bfloat16 *planes;
   long long plane, n8;
 };
-__global__ void __launch_bounds__(256) split3_pair_kernel(const SplitJob j0, const SplitJob j1, int *flag, int epoch) {
+__global__ void __launch_bounds__(256) split3_pair_kernel(const SplitJob j0, const SplitJob j1, int *flag) {
   bool bad = false;
   for (long long e = blockIdx.x * 256ll + threadIdx.x; e < j0.n8 + j1.n8; e += gridDim.x * 256ll) {
     const bool second = e >= j0.n8;
@@ -688,7 +687,7 @@ __global__ void __launch_bounds__(256) split3_pair_kernel(const SplitJob j0, con
     *reinterpret_cast<uint4 *>(J.planes + J.plane + 8 * i) = make_uint4(m[0], m[1], m[2], m[3]);
     *reinterpret_cast<uint4 *>(J.planes + 2 * J.plane + 8 * i) = make_uint4(l[0], l[1], l[2], l[3]);
   }
-  if (flag && bad) *flag = epoch;
+  if (flag && bad) *flag = 1;
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 t3_encode() {
@@ -762,7 +761,6 @@ cudaError_t t3_launch(const Gemm3Args &g, cudaStream_t s) {
   p.a32 = g.a32;
   p.b32 = g.b32;
   p.guard = g.out_mode == OUT_SQDIFF ? nullptr : g.guard;   // (the fallback stores its product)
-  p.epoch = g.epoch;
   p.bias = g.bias;
   p.relu = g.relu;
   // guarded: enough CTAs for the fallback's parts of the tiles
@@ -806,7 +804,7 @@ cudaError_t tc3_gemm_launch(const Gemm3Args &g, cudaStream_t s) {
 }
 
 cudaError_t split3_launch(const float *x, __nv_bfloat16 *planes, long long plane, long long n1, long long n1p,
-                          long long rest, double *partials, int num_partials, int *flag, int epoch, cudaStream_t s) {
+                          long long rest, double *partials, int num_partials, int *flag, cudaStream_t s) {
   if (n1 < 1 || n1p < n1 || n1p % 8 || rest < 1 || plane % 8 || plane < n1p * rest ||
       (reinterpret_cast<uintptr_t>(planes) & 15u) || (partials && num_partials < 1))
     return cudaErrorInvalidValue;
@@ -815,23 +813,23 @@ cudaError_t split3_launch(const float *x, __nv_bfloat16 *planes, long long plane
   int grid = partials ? num_partials
                       : static_cast<int>(std::min<long long>((total + 255) / 256, 8ll * device_sm_count()));
   if (partials) {
-    if (vec) split3_kernel<true, true><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, partials, flag, epoch);
-    else split3_kernel<false, true><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, partials, flag, epoch);
+    if (vec) split3_kernel<true, true><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, partials, flag);
+    else split3_kernel<false, true><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, partials, flag);
   } else {
-    if (vec) split3_kernel<true, false><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, nullptr, flag, epoch);
-    else split3_kernel<false, false><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, nullptr, flag, epoch);
+    if (vec) split3_kernel<true, false><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, nullptr, flag);
+    else split3_kernel<false, false><<<grid, 256, 0, s>>>(x, planes, plane, n1, n1p, rest, nullptr, flag);
   }
   return cudaGetLastError();
 }
 
 cudaError_t split3_pair_launch(const float *x, __nv_bfloat16 *planes, long long plane, long long n, const float *x2,
-                               __nv_bfloat16 *planes2, long long plane2, long long n2, int *flag, int epoch,
+                               __nv_bfloat16 *planes2, long long plane2, long long n2, int *flag,
                                cudaStream_t s) {
   if (n % 8 || n2 % 8 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x2)) & 15u))
     return cudaErrorInvalidValue;
   const SplitJob j0{x, planes, plane, n / 8}, j1{x2, planes2, plane2, n2 / 8};
   const int grid = static_cast<int>(std::min<long long>((j0.n8 + j1.n8 + 255) / 256, 8ll * device_sm_count()));
-  split3_pair_kernel<<<grid, 256, 0, s>>>(j0, j1, flag, epoch);
+  split3_pair_kernel<<<grid, 256, 0, s>>>(j0, j1, flag);
   return cudaGetLastError();
 }
 
