@@ -41,6 +41,7 @@
 #include "../../include/htgb.h"
 #include "common.cuh"
 #include "engine.h"
+#include "workspace.h"
 
 using namespace htgb;
 
@@ -69,12 +70,25 @@ ht_status_t fail(ht_status_t s, const std::string &msg) {
   } while (0)
 
 // ------------------------------------------------------------ workspace cache
-struct DeviceWorkspace {
-  void *ptr = nullptr;
-  size_t bytes = 0;
-};
 std::mutex g_ws_mutex;
-DeviceWorkspace g_ws[64];
+WorkspaceBlock g_ws[64];
+
+struct DeviceMemory {   // the allocator of grant_workspace
+  cudaStream_t st;
+  cudaError_t error = cudaSuccess;   // the last call that failed
+  bool ok(cudaError_t e) {
+    if (e == cudaSuccess) return true;
+    cudaGetLastError();
+    error = e;
+    return false;
+  }
+  bool room(size_t *free_bytes) {
+    size_t total = 0;
+    return ok(cudaMemGetInfo(free_bytes, &total));
+  }
+  bool allocate(void **p, size_t bytes) { return ok(cudaMalloc(p, bytes)); }
+  bool release(void *p) { return ok(cudaStreamSynchronize(st)) && ok(cudaDeviceSynchronize()) && ok(cudaFree(p)); }
+};
 
 // Per-device host state of the single-tensor call, guarded by g_ws_mutex:
 // a page-locked block that receives the call's status words in one copy (a
@@ -798,24 +812,42 @@ ht_status_t check_device() {
   return HT_OK;
 }
 
-ht_status_t acquire_workspace(size_t bytes, void **ptr, cudaStream_t st) {
+ht_status_t grant(WorkspaceBlock &w, size_t want, size_t least, bool optional, cudaStream_t st, Granted *got) {
+  DeviceMemory mem{st};
+  *got = grant_workspace(w, want, least, optional, mem);
+  if (*got != Granted::none) return HT_OK;
+  HT_CUDA(mem.error);
+  return fail(HT_ERR_OUT_OF_MEMORY, "no device memory for the workspace");
+}
+
+// `size` is called with a bool -- with or without what the call can do without --
+// and gives the bytes; the second time only where the block in hand is too small.
+template <class Size>
+ht_status_t acquire_workspace_for(Size &&size, void **ptr, size_t *bytes, bool *full, cudaStream_t st) {
   int dev = 0;
   HT_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(HT_ERR_INVALID_ARG, "device index out of range");
-  DeviceWorkspace &w = g_ws[dev];
-  if (w.bytes < bytes) {
-    if (w.ptr) {
-      HT_CUDA(cudaStreamSynchronize(st));
-      HT_CUDA(cudaDeviceSynchronize());
-      HT_CUDA(cudaFree(w.ptr));
-      w.ptr = nullptr;
-      w.bytes = 0;
+  WorkspaceBlock &w = g_ws[dev];
+  HT_TRY(size(true, bytes));
+  *full = true;
+  if (w.bytes < *bytes) {
+    size_t least = 0;
+    HT_TRY(size(false, &least));
+    least = std::min(least, *bytes);
+    Granted got;
+    HT_TRY(grant(w, *bytes, least, true, st, &got));
+    if (got == Granted::least) {
+      *full = false;
+      *bytes = least;
     }
-    HT_CUDA(cudaMalloc(&w.ptr, bytes));
-    w.bytes = bytes;
   }
   *ptr = w.ptr;
   return HT_OK;
+}
+
+ht_status_t acquire_workspace(size_t bytes, void **ptr, cudaStream_t st) {
+  bool full = true;
+  return acquire_workspace_for([&](bool, size_t *b) { *b = bytes; return HT_OK; }, ptr, &bytes, &full, st);
 }
 
 // ----------------------------------------------------------------- pipeline
@@ -2601,8 +2633,7 @@ ht_status_t ht_release_workspace(void) {
   if (dev >= 0 && dev < 64 && g_ws[dev].ptr) {
     HT_CUDA(cudaDeviceSynchronize());
     HT_CUDA(cudaFree(g_ws[dev].ptr));
-    g_ws[dev].ptr = nullptr;
-    g_ws[dev].bytes = 0;
+    g_ws[dev] = WorkspaceBlock{};
   }
   return HT_OK;
 }
@@ -2669,18 +2700,11 @@ ht_status_t ht_decompose(const float *x, const long *dims, int order, const ht_t
   std::lock_guard<std::mutex> lk(g_ws_mutex);
   CallArgs a{x, is_device_ptr(x), dims, order, U, B, (cfg.flags & HT_FLAG_COMPUTE_ERROR) != 0};
   size_t bytes = 0;
-  bool tc3 = true;   // FP32 products from operand planes (Ctx::tc3)
-  HT_TRY(sized_call_bytes(T, cfg, a, tc3, &bytes));
+  bool tc3 = true;   // FP32 products from operand planes (Ctx::tc3), where they have room
   void *ws = nullptr;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  ht_status_t got = acquire_workspace(bytes, &ws, st);
-  if (got == HT_ERR_OUT_OF_MEMORY && tc3) {   // no room for the planes: CUDA cores
-    cudaGetLastError();
-    tc3 = false;
-    HT_TRY(sized_call_bytes(T, cfg, a, tc3, &bytes));
-    got = acquire_workspace(bytes, &ws, st);
-  }
-  HT_TRY(got);
+  HT_TRY(acquire_workspace_for([&](bool planes, size_t *b) { return sized_call_bytes(T, cfg, a, planes, b); }, &ws,
+                               &bytes, &tc3, st));
   Ctx c;
   c.st = st;
   c.tc3 = tc3;
@@ -3267,23 +3291,19 @@ ht_status_t ht_reconstruct(const long *dims, int order, const ht_tree_t *tree, c
   };
   void *ws = nullptr;
   size_t bytes = 0;
-  bool tc3 = true;
-  auto acquire = [&]() -> ht_status_t {
-    Ctx d;
-    d.ar.dry = true;
-    d.tc3 = tc3;
-    HT_TRY(plan(d));
-    planes = d.planes;
-    bytes = d.ar.peak + (1 << 20);
-    return acquire_workspace(bytes, &ws, st);
-  };
-  ht_status_t got = acquire();
-  if (got == HT_ERR_OUT_OF_MEMORY) {   // no room for the planes: CUDA cores
-    cudaGetLastError();
-    tc3 = false;
-    got = acquire();
-  }
-  HT_TRY(got);
+  bool tc3 = true, planned = false;
+  HT_TRY(acquire_workspace_for(
+      [&](bool with_planes, size_t *b) -> ht_status_t {
+        Ctx d;
+        d.ar.dry = true;
+        d.tc3 = with_planes;
+        HT_TRY(plan(d));
+        planned = planned || d.planes;
+        *b = d.ar.peak + (1 << 20);
+        return HT_OK;
+      },
+      &ws, &bytes, &tc3, st));
+  planes = tc3 && planned;
   Ctx c;
   c.st = st;
   c.tc3 = tc3;
@@ -3402,20 +3422,18 @@ ht_status_t ht_evaluate(const long *dims, int order, const ht_tree_t *tree, cons
   };
   void *ws = nullptr;
   size_t bytes = 0;
-  auto acquire = [&]() -> ht_status_t {
-    Ctx d;
-    d.ar.dry = true;
-    HT_TRY(plan(d));
-    bytes = d.ar.peak + (1 << 20);
-    return acquire_workspace(bytes, &ws, st);
-  };
-  ht_status_t got = acquire();
-  if (got == HT_ERR_OUT_OF_MEMORY) {   // no room for the records: entry by entry
-    cudaGetLastError();
-    grouped = false;
-    got = acquire();
-  }
-  HT_TRY(got);
+  bool records = true;
+  HT_TRY(acquire_workspace_for(
+      [&](bool with_records, size_t *b) -> ht_status_t {
+        Ctx d;
+        d.ar.dry = true;
+        grouped = with_records;
+        HT_TRY(plan(d));
+        *b = d.ar.peak + (1 << 20);
+        return HT_OK;
+      },
+      &ws, &bytes, &records, st));
+  grouped = records;   // (without room for the records: entry by entry)
   Ctx c;
   c.st = st;
   c.ar.base = static_cast<char *>(ws);
@@ -3797,7 +3815,7 @@ void htd4(float *x, long a, long b, long c, long d, int *k, void *cublas_handle,
 namespace {
 
 std::mutex g_layer_mutex;
-DeviceWorkspace g_layer_ws[64];
+WorkspaceBlock g_layer_ws[64];
 int *g_layer_err[64];   // first 256 bytes of each device's layer workspace
 
 ht_status_t layer_shape(const ht_layer_shape_t *in, LayerShape *sh) {
@@ -3847,38 +3865,36 @@ ht_status_t layer_run(cudaStream_t st, bool tc, F &&plan) {
   HT_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(HT_ERR_INVALID_ARG, "device index out of range");
   bool tc3 = !tc;
-  size_t bytes = 0;
-  auto size = [&]() -> ht_status_t {
+  auto size = [&](bool planes, size_t *bytes) -> ht_status_t {
     Ctx d;
     d.ar.dry = true;
     d.tc = tc;
-    d.tc3 = tc3;
+    d.tc3 = planes;
     HT_TRY(plan(d));
-    bytes = d.ar.peak + 256 + (1 << 16);
+    *bytes = d.ar.peak + 256 + (1 << 16);
     return HT_OK;
   };
-  HT_TRY(size());
+  size_t bytes = 0;
+  HT_TRY(size(tc3, &bytes));
   std::lock_guard<std::mutex> lk(g_layer_mutex);
-  DeviceWorkspace &w = g_layer_ws[dev];
+  WorkspaceBlock &w = g_layer_ws[dev];
   if (w.bytes < bytes) {
-    if (w.ptr) {
+    size_t least = bytes;
+    if (tc3) HT_TRY(size(false, &least));
+    // a call being recorded cannot allocate: it does without the planes where it can
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HT_CUDA(cudaStreamIsCapturing(st, &cap));
+    void *const before = w.ptr;
+    Granted got;
+    least = std::min(least, bytes);
+    const ht_status_t s = grant(w, bytes, least, cap == cudaStreamCaptureStatusNone, st, &got);
+    g_layer_err[dev] = static_cast<int *>(w.ptr);   // (null where the old block is gone and there is no new one)
+    HT_TRY(s);
+    if (got == Granted::least) tc3 = false;
+    if (w.ptr != before) {
+      HT_CUDA(cudaMemset(w.ptr, 0, 256));
       HT_CUDA(cudaDeviceSynchronize());
-      HT_CUDA(cudaFree(w.ptr));
-      w.ptr = nullptr;
-      w.bytes = 0;
     }
-    cudaError_t e = cudaMalloc(&w.ptr, bytes);
-    if (e == cudaErrorMemoryAllocation && tc3) {   // no room for the operands' planes: CUDA cores
-      cudaGetLastError();
-      tc3 = false;
-      HT_TRY(size());
-      e = cudaMalloc(&w.ptr, bytes);
-    }
-    HT_CUDA(e);
-    HT_CUDA(cudaMemset(w.ptr, 0, 256));
-    HT_CUDA(cudaDeviceSynchronize());
-    w.bytes = bytes;
-    g_layer_err[dev] = static_cast<int *>(w.ptr);
   }
   Ctx c;
   c.st = st;
@@ -4112,13 +4128,12 @@ ht_status_t ht_layer_release(void) {
   HT_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(HT_ERR_INVALID_ARG, "device index out of range");
   std::lock_guard<std::mutex> lk(g_layer_mutex);
-  DeviceWorkspace &w = g_layer_ws[dev];
+  WorkspaceBlock &w = g_layer_ws[dev];
   if (w.ptr) {
     HT_CUDA(cudaDeviceSynchronize());
     HT_CUDA(cudaFree(w.ptr));
   }
-  w.ptr = nullptr;
-  w.bytes = 0;
+  w = WorkspaceBlock{};
   g_layer_err[dev] = nullptr;
   return HT_OK;
 }
