@@ -470,8 +470,8 @@ ht_status_t run_gemm(Ctx &c, const GemmReq &q) {
 // at 256, 130 at 128, 240 at 64; Grams of 260 to 397: 145 us against 198 at 64
 // although the 256-wide tiles compute 2.3 x the outputs), except where its tiles
 // are too few for the SMs and K too short to split: then narrower ones spread
-// the work.  Splits keep at least 16 K blocks each, so that the ring fills and a
-// short product needs no reduction launch.
+// the work.  Splits keep at least 16 K blocks each (four where the SMs would stay
+// idle), so that the ring fills and a short product needs no reduction launch.
 ht_status_t run_gemm3(Ctx &c, const GemmReq &q) {
   TileGen gen;
   auto make = [&](int bn) {
@@ -491,13 +491,24 @@ ht_status_t run_gemm3(Ctx &c, const GemmReq &q) {
     if (width > bn / 2 && 2 * work >= sm_count()) break;
   }
   const int nt = gen.count;
+  auto split = [&](long min_kb) {
+    const int most = std::max(1, sm_count() / nt);
+    const long per = std::max<long>((nkb + most - 1) / most, std::min<long>(nkb, min_kb));
+    return static_cast<int>((nkb + per - 1) / per);
+  };
   int splits = 1;
-  if (q.force_splits > 0) splits = q.force_splits;
-  else if (q.allow_split && nt < sm_count()) {
-    splits = std::max(1, sm_count() / nt);
-    long per = (nkb + splits - 1) / splits;
-    per = std::max<long>(per, std::min<long>(nkb, 16));
-    splits = static_cast<int>((nkb + per - 1) / per);
+  if (q.force_splits > 0) {
+    splits = q.force_splits;
+  } else if (q.allow_split && nt < sm_count()) {
+    splits = split(16);
+    // Where that leaves more than half of the SMs idle, a single CTA's chain of K
+    // blocks (~2.8 us each) is what the product takes: four to a split then, unless
+    // the chain is short and the sum over the splits of many tiles costs as much
+    // (512 x 1024, K = 512: 42 us a forward without, 47 with).  With 16, products of
+    // K = 1024 and few columns were slower than on the CUDA cores (layer 1024 ->
+    // 1024, batch 64: 64 us a forward against 55; 43 with four), and so were the
+    // Grams of tensors of 24 to 64 a mode (32^3: 384 us a call, 338; 312).
+    if (2ll * nt * splits < sm_count() && (nkb > 8 || 8 * nt < sm_count())) splits = split(4);
   }
   const bool partial = splits > 1 || q.out_mode == OUT_PARTIAL;
   const size_t mark = c.ar.off;
@@ -4014,7 +4025,11 @@ ht_status_t ht_layer_forward(const ht_layer_shape_t *shape, const float *u1, con
     __nv_bfloat16 *W16 = tc ? c.ar.take<__nv_bfloat16>(static_cast<size_t>(nin * nout)) : nullptr;
     __nv_bfloat16 *x16 = tc ? c.ar.take<__nv_bfloat16>(static_cast<size_t>(batch * nin)) : nullptr;
     Planes W3, x3;
-    if (c.tc3 && nin % 8 == 0) HT_TRY(reserve_planes(c, nin, nout, &W3));
+    // (short rows and few of them: x's planes are a launch more for a product that the
+    // CUDA cores form in a launch's time; 64 -> 64: 35 us a call against 38)
+    const bool tiny = (nin <= 64 || (nin <= 128 && batch <= 64)) &&
+                      static_cast<double>(nin) * nout * batch <= double(1 << 23);
+    if (c.tc3 && nin % 8 == 0 && !tiny && layer_weight_planes(sh, batch)) HT_TRY(reserve_planes(c, nin, nout, &W3));
     if (!P || !Q || !(W32 || W16) || (tc && !x16)) return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
     if (!c.dry()) {
       HT_CUDA(layer_pq_launch(sh, u1, u2, u3, b2, b1, P, Q, nullptr, c.st, c.nf));
@@ -4068,7 +4083,7 @@ ht_status_t ht_layer_backward(const ht_layer_shape_t *shape, const float *u1, co
       return fail(HT_ERR_OUT_OF_MEMORY, "layer workspace too small");
     Planes W3, x3, dy3;
     if (c.tc3 && nin % 8 == 0 && nout % 8 == 0) {
-      if (dx) HT_TRY(reserve_planes(c, nin, nout, &W3));
+      if (dx && layer_weight_planes(sh, batch)) HT_TRY(reserve_planes(c, nin, nout, &W3));
       HT_TRY(reserve_planes(c, nin, batch, &x3));
       HT_TRY(reserve_planes(c, nout, batch, &dy3));
     }

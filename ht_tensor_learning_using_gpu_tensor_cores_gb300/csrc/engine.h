@@ -479,6 +479,8 @@ cudaError_t layer_pq_launch(const LayerShape &sh, const float *u1, const float *
 // W (Nout x Nin, row-major) from P and Q, into W32 (FP32) or, when W32 is null, W16 (BF16)
 cudaError_t layer_weight_launch(const LayerShape &sh, const float *P, const float *Q, float *W32, __nv_bfloat16 *W16,
                                 __nv_bfloat16 *W3, long long plane, int *flag, cudaStream_t s);
+// Whether a product of `batch` columns with W is worth W's planes.
+bool layer_weight_planes(const LayerShape &sh, long long batch);
 // y[z, o] = act(y[z, o] + bias[o]) (bias may be null; act 0 identity, 1 ReLU)
 cudaError_t bias_act_launch(float *y, const float *bias, long long batch, long long nout, int act, cudaStream_t s);
 // Ranges of the batch whose partial column sums of dy layer_factor_grads_launch

@@ -18,6 +18,9 @@
 // u_j (N_j, M_j, r_j), b2 (r3, r4, r1), b1 (r1, r2), bias (M0, M1, M2).
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -212,6 +215,58 @@ __global__ void __launch_bounds__(kLayerThreads, RB < 64 ? 3 : 1) layer_weight_t
           bad |= KIND == W_PLANES && no_planes(v);
         }
     }
+  }
+  if (KIND == W_PLANES && bad) *flag = 1;
+}
+
+// The same W with P's rows as they are and Q's group of kWeightG m2 rows beside
+// them, both in shared memory, a thread with kWeightG sums for one input index: where
+// the padded rows above do not fit, or cost more than they save (layer_weight_form).
+// (12, 64, 32) -> (2, 8, 32) at rank 40: 0.43 ms a forward call, 1.9 with a thread
+// per entry of W.
+constexpr int kWeightG = 8;
+template <int KIND>
+__global__ void __launch_bounds__(kLayerThreads) layer_weight_packed_kernel(const LayerShape sh,
+                                                                            const float *__restrict__ P,
+                                                                            const float *__restrict__ Q,
+                                                                            const WeightOut W, int *flag) {
+  extern __shared__ __align__(16) float Ps[];   // NP x R1; behind it Qt: R1 x kWeightG x N2
+  const int N0 = sh.n[0], N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
+  const int R1 = sh.r1, B = N1 * M1, NP = N0 * N1;
+  const long long Nin = static_cast<long long>(NP) * N2;
+  const int groups = (M2 + kWeightG - 1) / kWeightG;
+  const int gi = blockIdx.x % groups, mm = blockIdx.x / groups, m1 = mm % M1, m0 = mm / M1;
+  const int m2_0 = gi * kWeightG, ng = min(kWeightG, M2 - m2_0);
+  float *Qt = Ps + static_cast<size_t>(NP) * R1;
+  for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
+    const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
+    Ps[e] = P[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r];
+  }
+  for (int e = threadIdx.x; e < R1 * kWeightG * N2; e += kLayerThreads) {
+    const int n2 = e % N2, g = (e / N2) % kWeightG, r = e / (N2 * kWeightG);
+    Qt[e] = g < ng ? Q[static_cast<long long>(n2 * M2 + m2_0 + g) * R1 + r] : 0.f;
+  }
+  __syncthreads();
+  const long long o0 = ((static_cast<long long>(m0) * M1 + m1) * M2 + m2_0) * Nin;
+  bool bad = false;
+  for (long long i = threadIdx.x; i < Nin; i += kLayerThreads) {
+    const int pr = static_cast<int>(i / N2), n2 = static_cast<int>(i - static_cast<long long>(pr) * N2);
+    float acc[kWeightG];
+#pragma unroll
+    for (int g = 0; g < kWeightG; ++g) acc[g] = 0.f;
+    const float *ps = Ps + static_cast<size_t>(pr) * R1;
+    for (int r = 0; r < R1; ++r) {
+      const float pv = ps[r];
+      const float *q = Qt + static_cast<size_t>(r) * kWeightG * N2 + n2;
+#pragma unroll
+      for (int g = 0; g < kWeightG; ++g) acc[g] = fmaf(pv, q[g * N2], acc[g]);
+    }
+#pragma unroll
+    for (int g = 0; g < kWeightG; ++g)
+      if (g < ng) {
+        put_weight<KIND>(W, o0 + g * Nin + i, acc[g]);
+        bad |= KIND == W_PLANES && no_planes(acc[g]);
+      }
   }
   if (KIND == W_PLANES && bad) *flag = 1;
 }
@@ -413,6 +468,68 @@ __global__ void __launch_bounds__(kLayerThreads) layer_dpq_kernel(const LayerSha
   for (int e = t; e < NP * R1; e += kLayerThreads) {
     const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
     dPo[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r] = dPs[r * NP + pr];
+  }
+}
+
+// The same pass without padding and without partial sums in shared memory, an
+// output of either product per thread and step, where the kernel above does not fit
+// or has too few pairs to keep its threads busy (layer_dpq_form).
+__global__ void __launch_bounds__(kLayerThreads) layer_dpq_packed_kernel(const LayerShape sh,
+                                                                         const float *__restrict__ dW,
+                                                                         const float *__restrict__ P,
+                                                                         const float *__restrict__ Q,
+                                                                         float *__restrict__ dP,
+                                                                         float *__restrict__ dQpart) {
+  extern __shared__ __align__(16) float sm[];
+  const int N0 = sh.n[0], N1 = sh.n[1], N2 = sh.n[2], M0 = sh.m[0], M1 = sh.m[1], M2 = sh.m[2];
+  const int R1 = sh.r1, B = N1 * M1, NP = N0 * N1, C = N2 * M2;
+  const int rs = N2 | 1;                             // odd stride between pairs: conflict-free column reads
+  const long long Nin = static_cast<long long>(NP) * N2;
+  const int chunks = gridDim.x / (M0 * M1);          // m2 ranges per (m0, m1): dP partials per range
+  const int blk = blockIdx.x / chunks, ch = blockIdx.x - blk * chunks, m1 = blk % M1, m0 = blk / M1;
+  const int mg = (M2 + chunks - 1) / chunks, m2_lo = ch * mg, m2_hi = min(M2, m2_lo + mg);
+  float *row = sm;                                   // NP x rs
+  float *Qs = row + static_cast<size_t>(NP) * rs;    // C x R1
+  float *Ps = Qs + static_cast<size_t>(C) * R1;      // NP x R1
+  float *dPs = Ps + static_cast<size_t>(NP) * R1;    // NP x R1
+  for (int e = threadIdx.x; e < C * R1; e += kLayerThreads) Qs[e] = Q[e];
+  for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
+    const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
+    Ps[e] = P[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r];
+    dPs[e] = 0.f;
+  }
+  for (int m2 = m2_lo; m2 < m2_hi; ++m2) {
+    __syncthreads();   // previous row fully consumed (and Qs / Ps written on the first pass)
+    const float *src = dW + ((static_cast<long long>(m0) * M1 + m1) * M2 + m2) * Nin;
+    for (long long i = threadIdx.x; i < Nin; i += kLayerThreads) {
+      const int pr = static_cast<int>(i / N2), n2 = static_cast<int>(i - static_cast<long long>(pr) * N2);
+      row[pr * rs + n2] = src[i];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
+      const int pr = e / R1, r = e - pr * R1;
+      const float *rw = row + pr * rs;
+      float s = dPs[e];
+      for (int n2 = 0; n2 < N2; ++n2) s = fmaf(rw[n2], Qs[(n2 * M2 + m2) * R1 + r], s);
+      dPs[e] = s;
+    }
+    for (int e = threadIdx.x; e < N2 * R1; e += kLayerThreads) {
+      const int r = e / N2, n2 = e - r * N2;
+      float s[4] = {0.f, 0.f, 0.f, 0.f};   // four independent chains, combined in a fixed order
+      int pr = 0;
+      for (; pr + 4 <= NP; pr += 4)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j] = fmaf(row[(pr + j) * rs + n2], Ps[(pr + j) * R1 + r], s[j]);
+      for (; pr < NP; ++pr) s[0] = fmaf(row[pr * rs + n2], Ps[pr * R1 + r], s[0]);
+      dQpart[(static_cast<long long>(blk) * C + (n2 * M2 + m2)) * R1 + r] = (s[0] + s[1]) + (s[2] + s[3]);
+    }
+  }
+  __syncthreads();
+  // chunks > 1: dP points at the partial buffer [chunks][A B R1]
+  float *dPo = dP + static_cast<long long>(ch) * (static_cast<long long>(sh.n[0]) * M0 * B * R1);
+  for (int e = threadIdx.x; e < NP * R1; e += kLayerThreads) {
+    const int pr = e / R1, r = e - pr * R1, n0 = pr / N1, n1 = pr - n0 * N1;
+    dPo[(static_cast<long long>(n0 * M0 + m0) * B + (n1 * M1 + m1)) * R1 + r] = dPs[e];
   }
 }
 
@@ -655,6 +772,10 @@ int layer_weight_rb(const LayerShape &sh) { return sh.r1 <= 16 ? 16 : (sh.r1 <= 
 size_t layer_weight_smem(const LayerShape &sh) {
   return sizeof(float) * (static_cast<size_t>(sh.n[0]) * sh.n[1] * layer_weight_rb(sh) + static_cast<size_t>(sh.n[2]) * 65);
 }
+size_t layer_weight_packed_smem(const LayerShape &sh) {
+  return sizeof(float) * (static_cast<size_t>(sh.n[0]) * sh.n[1] * sh.r1 +
+                          static_cast<size_t>(sh.r1) * kWeightG * sh.n[2]);
+}
 
 size_t layer_dpq_smem(const LayerShape &sh) {
   const size_t NP = static_cast<size_t>(sh.n[0]) * sh.n[1], C = static_cast<size_t>(sh.n[2]) * sh.m[2];
@@ -662,8 +783,59 @@ size_t layer_dpq_smem(const LayerShape &sh) {
   return sizeof(float) *
          (NP * (sh.n[2] | 1) + C * RP + NP * RP + 64 + NP * sh.r1 + static_cast<size_t>(kLayerThreads) * kDqRed);
 }
+size_t layer_dpq_packed_smem(const LayerShape &sh) {
+  const size_t NP = static_cast<size_t>(sh.n[0]) * sh.n[1], C = static_cast<size_t>(sh.n[2]) * sh.m[2];
+  return sizeof(float) * (NP * (sh.n[2] | 1) + C * sh.r1 + 2 * NP * sh.r1);
+}
 
 constexpr size_t kLayerSmemMax = 200 * 1024, kDpqSmemMax = 224 * 1024;
+
+// Which kernel forms W: the one whose estimated time (us) is the least.  The tiled
+// kernel's groups hold 64 / RB rows of W, so at ranks above 16, short N2 and many
+// pairs it mostly stages P; the packed one holds eight rows at any rank but has an
+// eighth of the threads' work per load; a thread per entry is for weights too few
+// to fill the SMs with blocks.  The coefficients are a fit to whole calls on 2617
+// shapes (8 to 4096 pairs, N2 of 2 to 800, ranks 2 to 64; median error 12 %); the
+// choice takes 1.01 x the best one's time on average, 1.6 x at worst, where tiled
+// wherever it fits took 1.22 x and up to 12 x ((12, 64, 8) -> (8, 8, 16) at rank 33:
+// 531 us against 133 packed, 217 by entry).
+enum WeightForm : int { WEIGHT_TILED, WEIGHT_PACKED, WEIGHT_ENTRIES };
+WeightForm layer_weight_form(const LayerShape &sh) {
+  const double pairs = static_cast<double>(sh.n[0]) * sh.n[1], n2 = sh.n[2], r = sh.r1;
+  const double m01 = static_cast<double>(sh.m[0]) * sh.m[1], entries = pairs * n2 * m01 * sh.m[2];
+  const int rb = layer_weight_rb(sh), G = 64 / rb;
+  auto waves = [&](int rows) { return std::ceil(m01 * ((sh.m[2] + rows - 1) / rows) / device_sm_count()); };
+  double tiled = 1e300, packed = 1e300;
+  if (layer_weight_smem(sh) <= kLayerSmemMax)
+    tiled = waves(G) * (8.7e-4 * pairs * rb + 7.9e-4 * pairs * n2 + 6.3e-3 * n2 + 0.084);
+  if (layer_weight_packed_smem(sh) <= kLayerSmemMax)
+    packed = waves(kWeightG) * (7.3e-4 * pairs * r + 2.0e-4 * pairs * n2 * r + 5.2e-4 * pairs * n2 + 6.1e-3 * r * n2);
+  const double by_entry = entries * (1.8e-6 * r + 6.7e-7);
+  if (tiled <= packed && tiled <= by_entry) return WEIGHT_TILED;
+  return packed <= by_entry ? WEIGHT_PACKED : WEIGHT_ENTRIES;
+}
+
+// Which of the two fused passes forms dP and dQ.  The tiled one keeps more outputs
+// per thread, but pads the ranks to four, holds 17 KB of partial sums and has work
+// for pairs x ranks / RT threads only.  Measured against each other over 597 shapes
+// (2 to 256 pairs, N2 of 8 to 128, ranks 3 to 64; whole backward calls, with the
+// tiled pass up to 2 x as fast at 256 pairs): the packed one is the faster
+//   * up to 48 pairs (median 1.02 to 1.1 x, up to 2.9 x where it also lets more
+//     CTAs share an SM: (4, 4, 128) -> (8, 8, 64) at rank 5, 1126 us unfused, 614),
+//   * up to 128 pairs where twice as many of its CTAs fit an SM, or where the blocks
+//     have a row or two each and their setup counts (1.04 to 1.15 x).
+// Where the tiled pass does not fit, the packed one is 2 to 4 x as fast as none.
+enum DpqForm : int { DPQ_NONE = 0, DPQ_TILED = 1, DPQ_PACKED = 2 };
+DpqForm layer_dpq_form(const LayerShape &sh) {
+  const size_t st = layer_dpq_smem(sh), sp = layer_dpq_packed_smem(sh);
+  if (sp > kLayerSmemMax) return st <= kDpqSmemMax ? DPQ_TILED : DPQ_NONE;
+  if (st > kDpqSmemMax) return DPQ_PACKED;
+  const long long pairs = static_cast<long long>(sh.n[0]) * sh.n[1];
+  const long long rows = static_cast<long long>(sh.m[0]) * sh.m[1] * sh.m[2];
+  auto ctas = [](size_t smem) { return std::min<size_t>(8, 227 * 1024 / (smem + 1024)); };   // that share an SM
+  const bool packed = pairs <= 48 || (pairs <= 128 && (ctas(sp) >= 2 * ctas(st) || rows <= 2 * device_sm_count()));
+  return packed ? DPQ_PACKED : DPQ_TILED;
+}
 
 template <class K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
@@ -671,12 +843,22 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
+// Where the packed kernel's blocks (eight rows of W each) leave SMs idle, the planes'
+// three more stores an entry lengthen it, and with few columns the CUDA cores'
+// product costs less than that: (12, 64, 32) -> (2, 8, 32) at rank 33, batch 64: 362
+// us a forward with planes, 337 without; batch 128: 374, 378; 256: 392, 497.
+bool layer_weight_planes(const LayerShape &sh, long long batch) {
+  const long long blocks = static_cast<long long>(sh.m[0]) * sh.m[1] * ((sh.m[2] + kWeightG - 1) / kWeightG);
+  return batch > 64 || blocks >= device_sm_count() || layer_weight_form(sh) != WEIGHT_PACKED;
+}
+
 template <int KIND>
 cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, const WeightOut &W, int *flag,
                           cudaStream_t s) {
   const long long total = static_cast<long long>(sh.n[0]) * sh.n[1] * sh.n[2] * sh.m[0] * sh.m[1] * sh.m[2];
-  const size_t smem = layer_weight_smem(sh);
-  if (smem <= kLayerSmemMax) {
+  const WeightForm form = layer_weight_form(sh);
+  if (form == WEIGHT_TILED) {
+    const size_t smem = layer_weight_smem(sh);
     const int rb = layer_weight_rb(sh), G = 64 / rb;
     const unsigned grid = static_cast<unsigned>(sh.m[0]) * sh.m[1] * ((sh.m[2] + G - 1) / G);
     auto launch = [&](auto kernel) -> cudaError_t {
@@ -688,6 +870,12 @@ cudaError_t weight_launch(const LayerShape &sh, const float *P, const float *Q, 
                           : rb == 32 ? launch(layer_weight_tiled_kernel<KIND, 32>)
                                      : launch(layer_weight_tiled_kernel<KIND, 64>);
     if (e != cudaSuccess) return e;
+  } else if (form == WEIGHT_PACKED) {
+    const size_t packed = layer_weight_packed_smem(sh);
+    const cudaError_t e = allow_smem(layer_weight_packed_kernel<KIND>, packed);
+    if (e != cudaSuccess) return e;
+    const unsigned grid = static_cast<unsigned>(sh.m[0]) * sh.m[1] * ((sh.m[2] + kWeightG - 1) / kWeightG);
+    layer_weight_packed_kernel<KIND><<<grid, kLayerThreads, packed, s>>>(sh, P, Q, W, flag);
   } else {
     layer_weight_kernel<KIND><<<grid_for_layer(total), kLayerThreads, 0, s>>>(sh, P, Q, W, flag);
   }
@@ -721,7 +909,7 @@ int layer_dpq_chunks(const LayerShape &sh) {
 }
 
 size_t layer_dq_part_count(const LayerShape &sh) {
-  if (layer_dpq_smem(sh) > kDpqSmemMax) return 0;
+  if (layer_dpq_form(sh) == DPQ_NONE) return 0;
   const size_t dq = static_cast<size_t>(sh.m[0]) * sh.m[1] * sh.n[2] * sh.m[2] * sh.r1;
   const int ch = layer_dpq_chunks(sh);
   const size_t dp = ch > 1 ? static_cast<size_t>(ch) * sh.n[0] * sh.m[0] * sh.n[1] * sh.m[1] * sh.r1 : 0;
@@ -736,10 +924,11 @@ cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, lon
   const int A = sh.n[0] * sh.m[0], B = sh.n[1] * sh.m[1], C = sh.n[2] * sh.m[2], NP = sh.n[0] * sh.n[1];
   const long long nout = static_cast<long long>(sh.m[0]) * sh.m[1] * sh.m[2];
   const int cchunks = layer_colsum_chunks(batch);
-  const size_t smem_dpq = layer_dpq_smem(sh);
+  const DpqForm form = layer_dpq_form(sh);
+  const size_t smem_dpq = form == DPQ_PACKED ? layer_dpq_packed_smem(sh) : layer_dpq_smem(sh);
   SumJobs sums{};
   cudaError_t e;
-  if (smem_dpq <= kDpqSmemMax && dQpart) {
+  if (form != DPQ_NONE && dQpart) {
     const int blocks = sh.m[0] * sh.m[1], ch = layer_dpq_chunks(sh);
     float *dPpart = dQpart + static_cast<size_t>(blocks) * C * sh.r1, *dPo = ch > 1 ? dPpart : dP;
     // ranks per thread: as many as leave every thread a pair
@@ -749,7 +938,8 @@ cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, lon
       kernel<<<static_cast<unsigned>(blocks * ch), kLayerThreads, smem_dpq, s>>>(sh, dW, P, Q, dPo, dQpart);
       return cudaGetLastError();
     };
-    if (NP * ((sh.r1 + 15) / 16) >= kLayerThreads) e = launch(layer_dpq_kernel<16>);
+    if (form == DPQ_PACKED) e = launch(layer_dpq_packed_kernel);
+    else if (NP * ((sh.r1 + 15) / 16) >= kLayerThreads) e = launch(layer_dpq_kernel<16>);
     else if (NP * ((sh.r1 + 7) / 8) >= kLayerThreads) e = launch(layer_dpq_kernel<8>);
     else e = launch(layer_dpq_kernel<4>);
     if (e != cudaSuccess) return e;

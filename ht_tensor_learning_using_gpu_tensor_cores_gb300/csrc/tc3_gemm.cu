@@ -207,10 +207,11 @@ __device__ __noinline__ void t3_fallback(const T3Params &p, const TileGen &gen, 
   constexpr int THREADS = F::C::THREADS;
   const int t = threadIdx.x, rg = t % 16, cg = t / 16;
   const long long ars = p.a32.rs, als = p.a32.ls, brs = p.b32.rs, bls = p.b32.ls;
-  // part w: columns [col0, col0 + SC) of item w / SUB's tile
+  // part w: columns [col0, col0 + SC) of item w % work's tile (first every item's
+  // first columns: a last tile may have no others)
   auto part = [&](int w, int &col0, int &tile_idx, int &split) {
-    const int item = w / F::SUB;
-    col0 = w % F::SUB * F::SC;
+    const int sub = w / p.work, item = w - sub * p.work;
+    col0 = sub * F::SC;
     tile_idx = item % p.num_tiles;
     split = item / p.num_tiles;
     return gen_tile(gen, tile_idx);
