@@ -338,7 +338,8 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
   uint64_t *empty = full + NSLOT;
   uint64_t *tfull = empty + NSLOT;
   uint64_t *tempty = tfull + 2;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 2);
+  uint64_t *idle = tempty + 2;   // an abandoned CTA's MMAs have ended
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(idle + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   if (p.guard && *p.guard != 0) {   // the same answer in every thread of the grid
@@ -359,6 +360,7 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
       mbar_init(&tfull[s], 1);
       mbar_init(&tempty[s], C::EW);
     }
+    mbar_init(idle, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
@@ -456,6 +458,14 @@ __global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
         umma_commit(&tfull[set]);
         ok = true;
        }
+      }
+      if (!ok) {
+        // a wait ran out with products under way: they read this CTA's shared memory
+        // and write its accumulators, which are freed only once they have ended (the
+        // drain warps wait for none of them)
+        int dummy = 0;
+        umma_commit(idle);
+        mbar_wait_bounded(idle, 0, &dummy);
       }
     }
     __syncwarp();
