@@ -206,6 +206,8 @@ def decompose(x, tree: DimTree, dims: Optional[Sequence[int]] = None, precision:
     precision="bf16": BF16 tcgen05 GEMMs with FP32 accumulation (the mixed path);
     precision="fp32": every product to FP32 accuracy (the plain path: CUDA cores,
     or three BF16 planes per operand on tensor cores).
+    report["path"] says which operands the products had: "tcgen05" BF16 ones,
+    "simt" FP32 ones (on CUDA cores or as planes).
     eig_iters: subspace iterations of the leaf solver (0: 10 on FP32, 6 on BF16).
     leaf_method="gram": leaf bases from the mode Grams (subspace iteration,
     eig_iters); "sketch": from the Gram-free range finder on X_(t)

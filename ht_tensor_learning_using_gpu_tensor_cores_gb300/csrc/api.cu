@@ -1471,6 +1471,16 @@ ht_status_t expand2(Ctx &c, const float *U0, long n0, int k0, const float *core,
     HT_CUDA(expand1_launch(U0, static_cast<int>(n0), k0, core, k1, k2, T, c.st));
     ++c.launches;
   }
+  // A short sum for few outputs: a thread each, where the product's 128 x 64 tiles
+  // are a few blocks (k1 = 8, 80 x 80 x 8: 4.5 us against 5.4; 130 x 130 x 8: 4.4,
+  // 5.3; 200 x 200 x 8: 5.8, 5.4; k1 = 16, 64 x 64 x 16: 5.8, 5.0).
+  if (k1 <= 10 && static_cast<double>(n0) * n1 * k2 * k1 <= 1.5e6) {
+    if (!c.dry()) {
+      HT_CUDA(expand2_small_launch(T, static_cast<int>(n0), k1, U1, static_cast<int>(n1), k2, W, c.st));
+      ++c.launches;
+    }
+    return HT_OK;
+  }
   // (ranks are at most 64: parse_tree)
   return nt_product(c, NtProduct{T, n0, static_cast<long long>(n0) * k1, U1, W, n0, static_cast<long long>(n0) * n1, n0,
                                  n1, k1, k2});
@@ -2403,7 +2413,6 @@ ht_status_t batch_enqueue(BatchState &b, const BatchLayout &L, cudaStream_t st, 
   HT_CUDA(tc_gram_grouped_launch(1, static_cast<char *>(b.grams) + tc_gram_item_bytes() * L.ngram[0], L.ngram[1], st));
   b.launches += (L.ngram[0] > 0) + (L.ngram[1] > 0);
   HT_TRY(batch_pass(b, L, 1, st, count, x, dims, order, trees, cfg, U, B, want_err, eig_ctas));
-  // external records: inside a capture they become event-record nodes of the graph
   HT_TRY(batch_phase_end(b, 0, st));
   // the wide problems (few, long) beside the narrow ones: their CTAs share the SMs
   if (L.nwide > 0) {

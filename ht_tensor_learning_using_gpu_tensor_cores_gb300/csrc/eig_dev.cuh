@@ -29,7 +29,7 @@ template <int N>
 HT_DEV void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Cyclic Jacobi on a symmetric s x s matrix held in shared memory (s <= SMAX),
-// 256 threads, round-robin ("circle method") ordering: every round rotates up
+// 256 or 1024 threads, round-robin ("circle method") ordering: every round rotates up
 // to s/2 disjoint pairs.  On return A is diagonal to FP32 rounding, V holds the
 // eigenvectors and order[] the indices by descending eigenvalue.  A2 is
 // scratch of the same shape.
@@ -45,9 +45,11 @@ HT_DEV void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : 
 // tiny late rotations c rounds to 1, and the plain c x - s y form would then
 // grow every column of V by s^2/2 per rotation (a 1e-5 loss of orthogonality
 // after ten sweeps); this form carries that second-order term explicitly.
-// The cosine uses a correctly rounded square root (an approximate one makes
-// every rotation slightly non-orthogonal, which the exact diagonal update then
-// turns into absolute errors on small eigenvalues).
+// The cosine is refined to FP32 rounding for its tangent (jac_choose): one that is
+// a few units off makes every rotation slightly non-orthogonal, which the exact
+// diagonal update then turns into absolute errors on small eigenvalues.  The
+// tangent itself may be a few units off: that only leaves a coupling below the
+// update's rounding, which the update sets to zero.
 //
 // Schedule.  Everything lives in position space: players (indices of the
 // matrix) sit at m positions, pair a is positions a ("top") and m - 1 - a

@@ -108,15 +108,15 @@ cudaError_t tc_prepare();
 // number of 64-wide K blocks of an operand pair (tcgen05 path)
 long tc_num_kblocks(const Operand &a);
 
-// FP32-accurate products on tcgen05 (tc3_gemm.cu): operands as three BF16
-// planes (`plane` elements apart, the first at Operand::ptr), tiles 128 x BN,
-// BN in {64, 128, 256} = gen.bn.
 // FP32 entries of an operand: row, l, r, z (see OpKind) at
 // row * rs + l * ls + r * rr + z * zs; l runs over len before r advances.
 struct Fp32Operand {
   const float *p = nullptr;
   long long rs = 0, ls = 0, rr = 0, zs = 0, len = 0;
 };
+// FP32-accurate products on tcgen05 (tc3_gemm.cu): operands as three BF16
+// planes (`plane` elements apart, the first at Operand::ptr), tiles 128 x BN,
+// BN in {64, 128, 256} = gen.bn.
 struct Gemm3Args {
   Operand a, b;
   // non-null guard: *guard != 0 (an operand entry had no planes, see
@@ -306,6 +306,9 @@ cudaError_t core_step2_launch(const float *T1, long long ldt, int nq, int kp, co
 // T[i0 + n0*(b + k1*c)] = sum_a U0[i0,a] core[a + k0*b + k0*k1*c]
 cudaError_t expand1_launch(const float *U0, int n0, int k0, const float *core, int k1, int k2, float *T,
                            cudaStream_t s);
+// W[i0 + n0*i1 + n0*n1*c] = sum_b T[i0 + n0*(b + k1*c)] U1[i1,b], a thread per output
+cudaError_t expand2_small_launch(const float *T, int n0, int k1, const float *U1, int n1, int k2, float *W,
+                                 cudaStream_t s);
 // C (m x n) = A (m x K) B (K x n), column-major
 cudaError_t matmul_nn_launch(const float *A, long long lda, const float *B, int ldb, float *C, long long ldc,
                              long long m, int n, int K, cudaStream_t s);

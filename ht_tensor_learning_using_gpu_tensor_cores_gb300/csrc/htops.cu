@@ -4,7 +4,7 @@
 // The reference reconstructs only the whole tensor, with cuBLAS calls on the
 // node bases (third_order_tensor_decompsition/CUDA/Optimized/htd_tensorcore.cu:
 // 295-331); it has no entry-wise evaluation.  Here the reconstruction is one
-// expansion of the interior node basis (small.cu expand2) and one NT product
+// expansion of the interior node basis (api.cu expand2) and one NT product
 // written straight into the column-major tensor.  Single entries are read from
 // precontracted matrices: every transfer tensor is folded with its parent's
 // and one child's factors into a matrix with one row per index of that child's

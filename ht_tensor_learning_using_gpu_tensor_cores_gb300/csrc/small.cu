@@ -494,6 +494,11 @@ HT_DEV void expand_step2_body(const float *__restrict__ T, int n0, int k1, const
     W[idx] = s;
   }
 }
+__global__ void expand_step2_kernel(const float *__restrict__ T, int n0, int k1, const float *__restrict__ U1, int n1,
+                                    int k2, float *__restrict__ W) {
+  expand_step2_body(T, n0, k1, U1, n1, k2, W, blockIdx.x, gridDim.x);
+}
+
 // C (m x n) = A (m x K) * B (K x n), column-major, small K and n
 __global__ void matmul_nn_kernel(const float *__restrict__ A, long long lda, const float *__restrict__ B, int ldb,
                                  float *__restrict__ C, long long ldc, long long m, int n, int K) {
@@ -945,6 +950,12 @@ cudaError_t core_step2_grouped_launch(const Step2Job *jobs_dev, const int *job_o
 cudaError_t expand1_launch(const float *U0, int n0, int k0, const float *core, int k1, int k2, float *T,
                            cudaStream_t s) {
   expand_step1_kernel<<<grid_for(static_cast<long long>(n0) * k1 * k2), 256, 0, s>>>(U0, n0, k0, core, k1, k2, T);
+  return cudaGetLastError();
+}
+
+cudaError_t expand2_small_launch(const float *T, int n0, int k1, const float *U1, int n1, int k2, float *W,
+                                 cudaStream_t s) {
+  expand_step2_kernel<<<grid_for(static_cast<long long>(n0) * n1 * k2), 256, 0, s>>>(T, n0, k1, U1, n1, k2, W);
   return cudaGetLastError();
 }
 

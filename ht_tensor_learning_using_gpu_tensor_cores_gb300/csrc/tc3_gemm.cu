@@ -325,8 +325,8 @@ __device__ __noinline__ void t3_fallback(const T3Params &p, const TileGen &gen, 
   }
 }
 
-template <int BN, int NSLOT, int MINB>
-__global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), MINB)
+template <int BN, int NSLOT>
+__global__ void __launch_bounds__((T3Cfg<BN, NSLOT>::THREADS), 1)
     tc3_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ T3Params p, const __grid_constant__ TileGen gen) {
   using C = T3Cfg<BN, NSLOT>;
@@ -744,12 +744,12 @@ long t3_kblocks(const Operand &o) {
 
 int tc3_grid(int work) { return std::min(work, device_sm_count()); }
 
-template <int BN, int NSLOT, int MINB>
+template <int BN, int NSLOT>
 cudaError_t t3_launch(const Gemm3Args &g, cudaStream_t s) {
   using C = T3Cfg<BN, NSLOT>;
   if (g.gen.bm != T3_BM || g.gen.bn != BN) return cudaErrorInvalidValue;
   static bool done[64] = {};
-  cudaError_t e = opt_in_smem(tc3_gemm_kernel<BN, NSLOT, MINB>, int(C::SMEM), done);
+  cudaError_t e = opt_in_smem(tc3_gemm_kernel<BN, NSLOT>, int(C::SMEM), done);
   if (e != cudaSuccess) return e;
   CUtensorMap ma, mb;
   if (!t3_map(g.a, g.a_plane, T3_BM, &ma) || !t3_map(g.b, g.b_plane, BN, &mb)) return cudaErrorInvalidValue;
@@ -777,7 +777,7 @@ cudaError_t t3_launch(const Gemm3Args &g, cudaStream_t s) {
   // guarded: enough CTAs for the fallback's parts of the tiles
   const int grid = p.guard ? int(std::min<long long>((long long)p.work * T3Fallback<BN, NSLOT>::SUB, device_sm_count()))
                            : tc3_grid(p.work);
-  tc3_gemm_kernel<BN, NSLOT, MINB><<<grid, C::THREADS, C::SMEM, s>>>(ma, mb, p, g.gen);
+  tc3_gemm_kernel<BN, NSLOT><<<grid, C::THREADS, C::SMEM, s>>>(ma, mb, p, g.gen);
   return cudaGetLastError();
 }
 
@@ -807,9 +807,9 @@ bool tc3_supported(const Operand &a, long long a_plane, const Operand &b, long l
 
 cudaError_t tc3_gemm_launch(const Gemm3Args &g, cudaStream_t s) {
   switch (g.gen.bn) {
-    case 64: return t3_launch<64, 8, 1>(g, s);
-    case 128: return t3_launch<128, 6, 1>(g, s);
-    case 256: return t3_launch<256, 4, 1>(g, s);
+    case 64: return t3_launch<64, 8>(g, s);
+    case 128: return t3_launch<128, 6>(g, s);
+    case 256: return t3_launch<256, 4>(g, s);
     default: return cudaErrorInvalidValue;
   }
 }
