@@ -1378,11 +1378,20 @@ struct NtProduct {
   long long batch;
 };
 
-// From these many multiply-adds the products of an HT expansion and the error
-// pass run from operand planes on tcgen05.  Below, the planes' launches (two of
-// ~3 us) and the persistent kernel's start (~5 us) cost more than the CUDA-core
-// kernels: gemm_nt_kernel does ~16 multiply-adds a ns, error_fused_kernel ~5.
-constexpr double kNt3MinMac = 2e8, kSq3MinMac = 5e7;
+// From these many multiply-adds a product runs from operand planes on tcgen05.
+// Below, the planes' launches and tensor maps (two of ~3 us each on the device, ~15
+// us of host time with the guard and its read-back) and the persistent kernel's
+// start cost more than the CUDA-core kernels take.
+//   Reconstruction, whole calls, CUDA cores against planes: 300^3 at rank 24 (6.5e8)
+//   134, 162 us; 350^3 rank 32 (1.4e9) 187, 189; 400^3 rank 24 (1.5e9) 208, 191; 500^3
+//   rank 8 (1e9) 205, 243, where both are bound by the output's bytes; 500^3 rank 16
+//   (2e9) 250, 237; 600^3 rank 8 (1.7e9) 324, 338.
+//   An expansion step beside other products of its call: 320 x 320 x 48 at rank 48
+//   (2.4e8) 3 us less on CUDA cores, 1024 x 1024 x 32 at rank 32 (1.1e9) 20 us more.
+//   Error pass: 200^3 at rank 16 (1.3e8) 578, 582 us a decomposition, 160^3 at rank
+//   48 (2e8) 879, 865, 256^3 at rank 48 (8e8) 1108, 1070.
+double nt3_min_mac(int k) { return k < 12 ? 2.5e9 : 1.4e9; }
+constexpr double kExpand3MinMac = 6e8, kSq3MinMac = 1.5e8;
 
 bool nt_with_planes(const Ctx &c, const NtProduct &p, double min_mac) {
   const bool dense = p.lda == p.m && (p.batch == 1 || p.sA == p.m * p.k);
@@ -1426,9 +1435,9 @@ ht_status_t nt_operands(Ctx &c, const NtProduct &p, Gemm3Args *g) {
   return HT_OK;
 }
 
-ht_status_t nt_product(Ctx &c, const NtProduct &p) {
+ht_status_t nt_product(Ctx &c, const NtProduct &p, double planes_min_mac) {
   const size_t mark = c.ar.off;
-  const bool planes = nt_with_planes(c, p, kNt3MinMac);
+  const bool planes = nt_with_planes(c, p, planes_min_mac);
   if (planes) {
     Gemm3Args g;
     HT_TRY(nt_operands(c, p, &g));
@@ -1482,8 +1491,10 @@ ht_status_t expand2(Ctx &c, const float *U0, long n0, int k0, const float *core,
     return HT_OK;
   }
   // (ranks are at most 64: parse_tree)
-  return nt_product(c, NtProduct{T, n0, static_cast<long long>(n0) * k1, U1, W, n0, static_cast<long long>(n0) * n1, n0,
-                                 n1, k1, k2});
+  return nt_product(c,
+                    NtProduct{T, n0, static_cast<long long>(n0) * k1, U1, W, n0, static_cast<long long>(n0) * n1, n0, n1,
+                              k1, k2},
+                    kExpand3MinMac);
 }
 
 // ||X - Xhat||_F^2 of an HT representation, into *dev_out (device double).
@@ -3257,7 +3268,7 @@ static ht_status_t reconstruct_core(Ctx &c, const Tree &T, const long *dims, int
       e.A = Wm; e.B = U[P.c]; e.m = e.ldc = np_; e.n = nc_; e.lda = np_ * nq_; e.sA = np_; e.sC = np_ * nc_;
       e.batch = nq_;
     }
-    HT_TRY(nt_product(c, e));
+    HT_TRY(nt_product(c, e, nt3_min_mac(e.k)));
   } else {
     const int t1 = T.left[0], t2 = T.right[0];
     const int k1 = T.rank[t1], k2 = T.rank[t2];
@@ -3275,7 +3286,7 @@ static ht_status_t reconstruct_core(Ctx &c, const Tree &T, const long *dims, int
       HT_CUDA(matmul_nn_launch(W12, R, B[0], k1, A12, R, R, k2, k1, c.st));
       ++c.launches;
     }
-    HT_TRY(nt_product(c, NtProduct{A12, R, 0, W34, out, R, 0, R, Cn, k2, 1}));
+    HT_TRY(nt_product(c, NtProduct{A12, R, 0, W34, out, R, 0, R, Cn, k2, 1}, nt3_min_mac(k2)));
   }
   c.ar.off = mark;
   return HT_OK;

@@ -127,7 +127,8 @@ def expansion(tr, U, B):
     return want.permute(*[order.index(m) for m in range(3)])
 
 
-@pytest.mark.parametrize("dims,r", [((301, 260, 397), 17), ((200, 150, 257), 64), ((40, 33, 65), 9)])
+# 1.4e9 multiply-adds take planes: two tensors above, one below
+@pytest.mark.parametrize("dims,r", [((301, 260, 397), 64), ((640, 321, 420), 17), ((40, 33, 65), 9)])
 @pytest.mark.parametrize("make", [ht.reference_tree_3d, ht.left_first_tree_3d, ht.middle_tree_3d])
 @pytest.mark.parametrize("e", [0, -116])
 def test_reconstruct(dims, r, make, e):
@@ -143,7 +144,8 @@ def test_reconstruct(dims, r, make, e):
     assert rel(X, expansion(tr, U, B)) < 3 * TOL   # core, both expansion steps, the product
 
 
-@pytest.mark.parametrize("dims", [(256, 200, 96), (181, 150, 203)])
+# (1.5e8 multiply-adds take planes)
+@pytest.mark.parametrize("dims", [(256, 200, 300), (301, 263, 203)])
 @pytest.mark.parametrize("make", [ht.reference_tree_3d, ht.left_first_tree_3d, ht.middle_tree_3d])
 def test_small_error_of_a_decomposition(dims, make):
     """An error of 1e-5, which an error delta of the expansion moves by delta^2 / 2e-5:
