@@ -3962,12 +3962,13 @@ ht_status_t layer_gemm(Ctx &c, const Operand &a32, const Operand &b32, const Ope
   if (rows >= 256 && cols >= 256) {
     // 256 x 256 tiles (two accumulators share every B stage) keep the tensor
     // pipe full where 128 x 256 ones leave it half idle (4096 x 4096 x 6400: 107
-    // against 204 us), so they are taken unless their last wave costs more
+    // against 204 us), so they are taken unless their last wave costs more.  Not
+    // where 128-row tiles are too few for the SMs: halving them again means splitting
+    // K in more parts of larger tiles, and the sum over the parts costs more than
+    // the MMAs gain (4096 x 1024 x 4096: 75 us a forward with 128 rows, 127 with 256)
     const long long t1 = ((rows + 127) / 128) * ((cols + 255) / 256), t2 = ((rows + 255) / 256) * ((cols + 255) / 256);
     auto waves = [](long long t) { return t < sm_count() ? 1.0 : double((t + sm_count() - 1) / sm_count()); };
-    // (too few tiles for the SMs: only where K is long enough to split)
-    const bool few = t1 < sm_count();
-    if (few ? t2 * (a16.ptr ? tc_num_kblocks(a16) / 16 : 0) >= sm_count() : 2.1 * waves(t2) <= 1.9 * waves(t1)) q.mt_tc = 2;
+    if (t1 >= sm_count() && 2.1 * waves(t2) <= 1.9 * waves(t1)) q.mt_tc = 2;
   }
   q.bn_simt = cols > 64 ? 128 : 64;
   q.tiles_kind = TILES_GRID;

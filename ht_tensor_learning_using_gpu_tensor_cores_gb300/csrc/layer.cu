@@ -736,8 +736,12 @@ HT_DEV void layer_db1_body(const LayerShape &sh, const float *__restrict__ dQ, c
   }
 }
 
+// Registers: du2's RB loads of T1 should all be in flight.  Left to itself the
+// compiler gives RB = 32 64 registers, and the kernel then took up to twice as long
+// as one of du2 alone (A = 256, B = 64, rank 32: 287 us a backward, 176 with 128
+// registers).
 template <int RB>   // rank bound: R2, R4 <= RB
-__global__ void __launch_bounds__(kLayerThreads) layer_grads_kernel(const LayerShape sh, const float *__restrict__ u2,
+__global__ void __launch_bounds__(kLayerThreads, RB == 16 ? 4 : 2) layer_grads_kernel(const LayerShape sh, const float *__restrict__ u2,
                                                                     const float *__restrict__ u3,
                                                                     const float *__restrict__ b1,
                                                                     const float *__restrict__ T1,
@@ -904,7 +908,9 @@ int layer_colsum_chunks(long long batch) {
 
 int layer_dpq_chunks(const LayerShape &sh) {
   const int blocks = sh.m[0] * sh.m[1];
-  int ch = (3 * device_sm_count() / 2 + blocks - 1) / blocks;   // two blocks an SM, in one wave
+  // a CTA and a half an SM; two of the packed form, of which more share one
+  const int ctas = layer_dpq_form(sh) == DPQ_PACKED ? 2 * device_sm_count() : 3 * device_sm_count() / 2;
+  int ch = (ctas + blocks - 1) / blocks;
   return ch < 1 ? 1 : (ch > sh.m[2] ? sh.m[2] : ch);
 }
 
@@ -971,6 +977,7 @@ cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, lon
   if (rb <= 16) grads(layer_grads_kernel<16>);
   else if (rb <= 32) grads(layer_grads_kernel<32>);
   else grads(layer_grads_kernel<kLayerMaxRank>);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const long long du1_blocks = (static_cast<long long>(A) * sh.r3 + kLayerThreads / 32 - 1) / (kLayerThreads / 32);
   const long long db2_blocks =
       (static_cast<long long>(sh.r3) * sh.r4 * sh.r1 + kLayerThreads - 1) / kLayerThreads;
