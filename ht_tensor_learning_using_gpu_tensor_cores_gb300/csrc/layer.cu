@@ -736,25 +736,34 @@ HT_DEV void layer_db1_body(const LayerShape &sh, const float *__restrict__ dQ, c
   }
 }
 
-// Registers: du2's RB loads of T1 should all be in flight.  Left to itself the
-// compiler gives RB = 32 64 registers, and the kernel then took up to twice as long
-// as one of du2 alone (A = 256, B = 64, rank 32: 287 us a backward, 176 with 128
-// registers).
 template <int RB>   // rank bound: R2, R4 <= RB
-__global__ void __launch_bounds__(kLayerThreads, RB == 16 ? 4 : 2) layer_grads_kernel(const LayerShape sh, const float *__restrict__ u2,
-                                                                    const float *__restrict__ u3,
-                                                                    const float *__restrict__ b1,
-                                                                    const float *__restrict__ T1,
-                                                                    const float *__restrict__ dP,
-                                                                    const float *__restrict__ dQ,
-                                                                    float *__restrict__ dT1, float *__restrict__ du2,
-                                                                    float *__restrict__ du3, float *__restrict__ db1,
-                                                                    int nb_du2, int nb_dt1) {
+HT_DEV void layer_grads_body(const LayerShape &sh, const float *__restrict__ u2, const float *__restrict__ u3,
+                             const float *__restrict__ b1, const float *__restrict__ T1, const float *__restrict__ dP,
+                             const float *__restrict__ dQ, float *__restrict__ dT1, float *__restrict__ du2,
+                             float *__restrict__ du3, float *__restrict__ db1, int nb_du2, int nb_dt1) {
   __shared__ float smem[2 * kDtChunk * kLayerMaxRank];
   const int blk = blockIdx.x;
   if (blk < nb_du2) layer_du2_body<RB>(sh, dP, T1, du2, blk, smem);
   else if (blk < nb_du2 + nb_dt1) layer_dt1_body(sh, u2, b1, dP, dQ, dT1, du3, blk - nb_du2, smem);
   else layer_db1_body<RB>(sh, dQ, u3, db1, blk - nb_du2 - nb_dt1, smem);
+}
+
+template <int RB>
+__global__ void __launch_bounds__(kLayerThreads) layer_grads_kernel(
+    const LayerShape sh, const float *__restrict__ u2, const float *__restrict__ u3, const float *__restrict__ b1,
+    const float *__restrict__ T1, const float *__restrict__ dP, const float *__restrict__ dQ, float *__restrict__ dT1,
+    float *__restrict__ du2, float *__restrict__ du3, float *__restrict__ db1, int nb_du2, int nb_dt1) {
+  layer_grads_body<RB>(sh, u2, u3, b1, T1, dP, dQ, dT1, du2, du3, db1, nb_du2, nb_dt1);
+}
+// du2's RB loads of T1 should all be in flight.  Left to itself the compiler gives
+// RB = 32 64 registers, and the kernel then took up to twice as long (A = 256, B = 64,
+// rank 32: 287 us a backward, 176 with the 128 registers of two CTAs an SM); at 16
+// the bound only costs (up to 1.2 x), at 64 it changes nothing.
+__global__ void __launch_bounds__(kLayerThreads, 2) layer_grads32_kernel(
+    const LayerShape sh, const float *__restrict__ u2, const float *__restrict__ u3, const float *__restrict__ b1,
+    const float *__restrict__ T1, const float *__restrict__ dP, const float *__restrict__ dQ, float *__restrict__ dT1,
+    float *__restrict__ du2, float *__restrict__ du3, float *__restrict__ db1, int nb_du2, int nb_dt1) {
+  layer_grads_body<32>(sh, u2, u3, b1, T1, dP, dQ, dT1, du2, du3, db1, nb_du2, nb_dt1);
 }
 
 }  // namespace
@@ -975,7 +984,7 @@ cudaError_t layer_factor_grads_launch(const LayerShape &sh, const float *dW, lon
     kernel<<<grid, kLayerThreads, 0, s>>>(sh, u2, u3, b1, T1, dP, dQ, dT1, du2, du3, db1, B, A + du3_blocks);
   };
   if (rb <= 16) grads(layer_grads_kernel<16>);
-  else if (rb <= 32) grads(layer_grads_kernel<32>);
+  else if (rb <= 32) grads(layer_grads32_kernel);
   else grads(layer_grads_kernel<kLayerMaxRank>);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const long long du1_blocks = (static_cast<long long>(A) * sh.r3 + kLayerThreads / 32 - 1) / (kLayerThreads / 32);
