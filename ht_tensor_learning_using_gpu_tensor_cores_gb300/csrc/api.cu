@@ -448,10 +448,10 @@ ht_status_t run_gemm(Ctx &c, const GemmReq &q) {
   ++c.launches;
   if (partial && !q.part_ext) {
     HT_CUDA(reduce_partials_launch(part, gen, splits, bn, q.out, q.ld_out,
-                                   (q.symmetric ? 1 : 0) | (q.accumulate ? 2 : 0), c.st));
+                                   (q.symmetric ? 1 : 0) | (q.accumulate ? 2 : 0), c.st, q.bias, q.relu ? 1 : 0));
     ++c.launches;
   }
-  if (!fused && (q.bias || q.relu)) {   // y row-major = this output's columns
+  if (!fused && !partial && (q.bias || q.relu)) {   // y row-major = this output's columns
     HT_CUDA(bias_act_launch(q.out, q.bias, q.t_n, q.ld_out, q.relu ? 1 : 0, c.st));
     ++c.launches;
   }
@@ -540,12 +540,8 @@ ht_status_t run_gemm3(Ctx &c, const GemmReq &q) {
   ++c.launches;
   if (partial && !q.part_ext) {
     HT_CUDA(reduce_partials_launch(part, gen, splits, bn, q.out, q.ld_out,
-                                   (q.symmetric ? 1 : 0) | (q.accumulate ? 2 : 0), c.st));
+                                   (q.symmetric ? 1 : 0) | (q.accumulate ? 2 : 0), c.st, q.bias, q.relu ? 1 : 0));
     ++c.launches;
-    if (q.bias || q.relu) {
-      HT_CUDA(bias_act_launch(q.out, q.bias, q.t_n, q.ld_out, q.relu ? 1 : 0, c.st));
-      ++c.launches;
-    }
   }
   c.ar.off = mark;
   return HT_OK;

@@ -171,9 +171,11 @@ long simt_k_total(const Operand &a);
 // Sum split-K partial tiles ([splits][tiles][gen.bm][bn]) into out.  symmetric
 // bit 0 clear: plain column-major tiles; set: a symmetric Gram (tiles on/above
 // the diagonal, mirrored into the lower triangle).  Bit 1: add the sums to what
-// out holds instead of overwriting it (a Gram accumulated over slabs).
+// out holds instead of overwriting it (a Gram accumulated over slabs).  bias (of
+// row r, or null) and ReLU: plain tiles only.
 cudaError_t reduce_partials_launch(const float *partial, const TileGen &gen, int splits, int bn, float *out,
-                                   long long ld_out, int symmetric, cudaStream_t s);
+                                   long long ld_out, int symmetric, cudaStream_t s, const float *bias = nullptr,
+                                   int relu = 0);
 TileGen make_rows_gen(long long rows, int cols, int bn);
 TileGen make_slabs_gen(long long L, long long R, int cols, int bn);
 // rows x cols output in 128 x bn tiles (TILES_GRID); false when the tile count overflows

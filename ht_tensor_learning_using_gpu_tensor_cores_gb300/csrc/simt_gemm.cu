@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(256, 2) simt_gemm_grouped_kernel(const SParams
 // flight when there are few outputs and many splits (small Grams).
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const float *__restrict__ part, const TileGen gen,
                                                               int num_tiles, int splits, int bn, int groups,
-                                                              float *__restrict__ out, long long ld, int symmetric) {
+                                                              float *__restrict__ out, long long ld, int symmetric,
+                                                              const float *__restrict__ bias, int relu) {
   __shared__ float red[256];
   const int nout = 256 / groups;
   const int o = threadIdx.x % nout, g = threadIdx.x / nout;
@@ -321,7 +322,10 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float *__res
         const long long gr = tl.out_row + row, gc = tl.out_col + col;
         const bool acc = (symmetric & 2) != 0;   // add to what out holds
         if (!(symmetric & 1)) {
-          out[gr + ld * gc] = acc ? out[gr + ld * gc] + s : s;
+          float v = acc ? out[gr + ld * gc] + s : s;
+          if (bias) v += bias[gr];
+          if (relu) v = fmaxf(v, 0.f);
+          out[gr + ld * gc] = v;
         } else if (gc >= gr) {   // the mirror element is produced by the tile holding (gc, gr)
           const long long a = gr + ld * gc, b = gc + ld * gr;
           const float v = acc ? out[a] + s : s;
@@ -458,7 +462,7 @@ cudaError_t simt_gemm_launch(const GemmArgs &g, int bn, cudaStream_t s) {
 }
 
 cudaError_t reduce_partials_launch(const float *partial, const TileGen &gen, int splits, int bn, float *out,
-                                   long long ld_out, int symmetric, cudaStream_t s) {
+                                   long long ld_out, int symmetric, cudaStream_t s, const float *bias, int relu) {
   const long long total = static_cast<long long>(gen.bm) * bn * gen.count;
   // split groups: about 8 partials per thread, at most 8 groups
   int groups = 1;
@@ -467,7 +471,8 @@ cudaError_t reduce_partials_launch(const float *partial, const TileGen &gen, int
   long long blocks = (total + nout - 1) / nout;
   const long long cap = 16ll * device_sm_count();
   const int grid = static_cast<int>(blocks < cap ? blocks : cap);
-  reduce_partials_kernel<<<grid, 256, 0, s>>>(partial, gen, gen.count, splits, bn, groups, out, ld_out, symmetric);
+  reduce_partials_kernel<<<grid, 256, 0, s>>>(partial, gen, gen.count, splits, bn, groups, out, ld_out, symmetric,
+                                           bias, relu);
   return cudaGetLastError();
 }
 
